@@ -968,16 +968,11 @@ void canonicalize(qse_state* st)
 {
     materialize(st);
     st->touch();
-    // restore logical == physical with physical qubit swaps (each a half sweep)
-    for (uint32_t q = 0; q < st->n; ++q) {
-        if (st->perm[q] == q) continue;
-        // find the logical qubit r currently sitting on physical q
-        uint32_t r = q;
-        for (uint32_t s = 0; s < st->n; ++s)
-            if (st->perm[s] == q) r = s;
-        launch_swap(st, q, st->perm[q]);
-        std::swap(st->perm[q], st->perm[r]);
-    }
+    // restore logical == physical: one in-place pass, two when the map is not
+    // made of swaps alone
+    if (st->identity_perm()) return;
+    permute_bits(st, st->perm);
+    for (uint32_t q = 0; q < st->n; ++q) st->perm[q] = q;
 }
 
 // ---------------------------------------------------------------- observables

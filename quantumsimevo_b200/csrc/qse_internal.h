@@ -174,6 +174,7 @@ void launch_ry(qse_state* st, uint32_t q, double c, double s);
 void launch_rz(qse_state* st, uint32_t q, double c0, double s0, double c1, double s1);
 void launch_cnot(qse_state* st, uint32_t c, uint32_t t);
 void launch_swap(qse_state* st, uint32_t q0, uint32_t q1);
+void permute_bits(qse_state* st, const uint32_t* perm);              // new[i] = old[perm(i)], index bit q read at perm[q]
 void launch_init_zero_state(qse_state* st);                          // write |0..0> now
 void mark_basis(qse_state* st, uint64_t phys_index);                 // lazy |phys_index>
 void mark_zero(qse_state* st);       // reset without writing: lazy |0..0>
