@@ -176,7 +176,8 @@ __device__ uint64_t block_scan_add(uint64_t v, uint64_t& excl, uint64_t* sh)
     return total;
 }
 
-// block_scan_add on integer-valued doubles; exact while the sums stay below 2^53
+// block_scan_add on integer-valued doubles; every prefix below 2^53 is exact
+// (also where later values are not: the exclusive prefix is never a difference)
 __device__ double block_scan_addd(double v, double& excl, double* sh)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -199,7 +200,8 @@ __device__ double block_scan_addd(double v, double& excl, double* sh)
         sh[64] = run;
     }
     __syncthreads();
-    excl = sh[32 + warp] + (inc - v);
+    const double before = __shfl_up_sync(0xffffffffu, inc, 1);
+    excl = sh[32 + warp] + (lane ? before : 0.0);
     const double total = sh[64];
     __syncthreads();
     return total;
@@ -264,7 +266,8 @@ __device__ void block_scan_maps(uint64_t t0, uint64_t t1, uint64_t& ex0, uint64_
 __device__ __forceinline__ double block_exact(uint32_t cnt, double c_in, double* out, uint64_t* sh, double* stage)
 {
     __shared__ double s_c;
-    __shared__ int s_t;
+    __shared__ int s_t, s_tie;
+    constexpr uint32_t kRun = 64;   // about 0.3 us of dependent additions
     const uint32_t tid = threadIdx.x;
     uint32_t pos = 0;
     double c = c_in;
@@ -320,103 +323,131 @@ __device__ __forceinline__ double block_exact(uint32_t cnt, double c_in, double*
             }
         }
     }
-    // general path (the fast path writes stage only when it returns)
-    double p[kEPT];
-#pragma unroll
-    for (int j = 0; j < kEPT; ++j) p[j] = stage[tid * kPad + j];
+    // One step per binade: the elements from pos up to the first that leaves the
+    // running sum's binade (t) are summed on its grid at once, then up to kRun
+    // elements from t on by real FP64 additions, the reference's own (a sum that
+    // starts near zero doubles every few elements, so the run takes several
+    // binades at once).  The grid sums run on doubles when no element before t
+    // ties: prefixes below 2^53 are exact whatever follows them.  (The element
+    // maps unrolled over 16 elements made the code of one step so long that
+    // fetching it dominated: 10 us a step, now about 2.)
+    bool seq = c == 0.0;   // a zero sum: start with a run
     while (pos < cnt) {
-        const int e = epoch_of(c);
-        const double G = ldexp(1.0, e - 52);
-        const uint64_t C = uint64_t(ldexp(c, 52 - e));
-        const Grid g = grid_of(e);
-        // this thread's element maps over its elements >= pos (even-parity
-        // offsets kept; a tie anywhere sends the block to the general path,
-        // which recomputes both offsets)
-        uint64_t Ci[kEPT];
-        int bad = kBS;
-        bool pure = true;
-        uint64_t tsum = 0;
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j) {
-            uint32_t i = tid * kEPT + j;
-            uint64_t a0 = 0, a1 = 0;
-            if (i >= pos && i < cnt) {
-                if (!elem_map_g(p[j], g, a0, a1) && bad == kBS) bad = int(i);
+        uint32_t t = pos;
+        if (!seq) {
+            const int e = epoch_of(c);
+            const double G = ldexp(1.0, e - 52);
+            const Grid g = grid_of(e);
+            if (tid == 0) {
+                s_t = int(cnt);
+                s_tie = int(cnt);
             }
-            Ci[j] = a0;
-            pure = pure && a0 == a1;
-            tsum += a0;
+            __syncthreads();
+            bool fast = g.fast != 0;
+            double q[kEPT];
+            if (fast) {
+                double tsum = 0.0;
+                int first = int(cnt), tie = int(cnt);
+#pragma unroll
+                for (int j = kEPT - 1; j >= 0; --j) {
+                    const uint32_t i = tid * kEPT + j;
+                    const double pj = stage[tid * kPad + j];
+                    const bool in = i >= pos && i < cnt;
+                    const double x = pj * g.scale;
+                    const double r = rint(x);
+                    const double df = x - r;
+                    if (in && !(pj < g.limit)) first = int(i);
+                    if (in && (df == 0.5 || df == -0.5)) tie = int(i);
+                    q[j] = in ? r : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < kEPT; ++j) tsum += q[j];
+                double ex;
+                block_scan_addd(tsum, ex, reinterpret_cast<double*>(sh));
+                double run = c * g.scale + ex;
+#pragma unroll
+                for (int j = 0; j < kEPT; ++j) {
+                    run += q[j];
+                    q[j] = run;
+                }
+#pragma unroll
+                for (int j = kEPT - 1; j >= 0; --j) {
+                    const int i = int(tid * kEPT) + j;
+                    if (i >= int(pos) && i < first && q[j] >= 0x1p53) first = i;
+                }
+                if (first < int(cnt)) atomicMin(&s_t, first);
+                if (tie < int(cnt)) atomicMin(&s_tie, tie);
+                __syncthreads();
+                fast = s_tie >= s_t;   // a tie at t itself is added for real
+                t = uint32_t(s_t);
+            }
+            if (fast) {
+#pragma unroll
+                for (int j = 0; j < kEPT; ++j) {
+                    const uint32_t i = tid * kEPT + j;
+                    if (i < pos || i >= t) continue;
+                    if (out) stage[tid * kPad + j] = q[j] * G;
+                    if (i + 1 == t) s_c = q[j] * G;   // c_{t-1}
+                }
+            } else {
+                // ties before t, or a subnormal sum's grid: parity maps, loops kept rolled
+                __syncthreads();   // s_t above is read by every thread
+                if (tid == 0) s_t = int(cnt);
+                const uint64_t C = uint64_t(ldexp(c, 52 - e));
+                uint64_t t0 = 0, t1 = 0;
+                int first = int(cnt);
+                auto step = [&](uint32_t j, uint64_t& m0, uint64_t& m1) {
+                    uint64_t a0, a1, r0, r1;
+                    const bool in = elem_map_g(stage[tid * kPad + j], g, a0, a1);
+                    compose(m0, m1, a0, a1, r0, r1);
+                    m0 = r0;
+                    m1 = r1;
+                    return in;
+                };
+                const uint32_t j0 = pos > tid * kEPT ? min(pos - tid * kEPT, uint32_t(kEPT)) : 0u;
+                const uint32_t j1 = cnt > tid * kEPT ? min(cnt - tid * kEPT, uint32_t(kEPT)) : 0u;
+#pragma unroll 1
+                for (uint32_t j = j0; j < j1; ++j)
+                    if (!step(j, t0, t1)) first = min(first, int(tid * kEPT + j));
+                uint64_t ex0, ex1;
+                block_scan_maps(t0, t1, ex0, ex1, sh);
+                uint64_t run0 = ex0, run1 = ex1;
+#pragma unroll 1
+                for (uint32_t j = j0; j < j1; ++j) {
+                    step(j, run0, run1);
+                    if (C + ((C & 1) ? run1 : run0) >= kTwo53) first = min(first, int(tid * kEPT + j));
+                }
+                if (first < int(cnt)) atomicMin(&s_t, first);
+                __syncthreads();
+                t = uint32_t(s_t);
+                run0 = ex0;
+                run1 = ex1;
+#pragma unroll 1
+                for (uint32_t j = j0; j < j1 && tid * kEPT + j < t; ++j) {
+                    step(j, run0, run1);
+                    const double v = double(C + ((C & 1) ? run1 : run0)) * G;
+                    if (out) stage[tid * kPad + j] = v;
+                    if (tid * kEPT + j + 1 == t) s_c = v;
+                }
+            }
+            if (tid == 0 && t == pos) s_c = c;   // no element on this grid
+        } else if (tid == 0) {
+            s_c = c;
         }
-        int first = bad;
-        if (__syncthreads_and(pure)) {
-            // no ties anywhere: every map is a translation and prefixes are sums
-            uint64_t ex;
-            block_scan_add(tsum, ex, sh);
-            uint64_t run = C + ex;
-#pragma unroll
-            for (int j = 0; j < kEPT; ++j) {
-                run += Ci[j];
-                Ci[j] = run;
-                uint32_t i = tid * kEPT + j;
-                if (i >= pos && i < cnt && run >= kTwo53 && int(i) < first) first = int(i);
-            }
-        } else {
-            uint64_t t0 = 0, t1 = 0;
-#pragma unroll
-            for (int j = 0; j < kEPT; ++j) {
-                uint64_t a0 = 0, a1 = 0, r0, r1;
-                const uint32_t i = tid * kEPT + j;
-                if (i >= pos && i < cnt) elem_map_g(p[j], g, a0, a1);
-                compose(t0, t1, a0, a1, r0, r1);
-                t0 = r0;
-                t1 = r1;
-            }
-            uint64_t ex0, ex1;
-            block_scan_maps(t0, t1, ex0, ex1, sh);
-            // running values; first index that reaches 2^53 or is flagged
-            uint64_t run0 = ex0, run1 = ex1;
-#pragma unroll
-            for (int j = 0; j < kEPT; ++j) {
-                uint64_t a0 = 0, a1 = 0, r0, r1;
-                const uint32_t i = tid * kEPT + j;
-                if (i >= pos && i < cnt) elem_map_g(p[j], g, a0, a1);
-                compose(run0, run1, a0, a1, r0, r1);
-                run0 = r0;
-                run1 = r1;
-                uint64_t v = C + ((C & 1) ? run1 : run0);
-                Ci[j] = v;
-                if (i >= pos && i < cnt && v >= kTwo53 && int(i) < first) first = int(i);
-            }
-        }
-        if (tid == 0) s_t = int(cnt);
         __syncthreads();
-        if (first < int(cnt)) atomicMin(&s_t, first);
-        __syncthreads();
-        const uint32_t t = uint32_t(s_t);
-        // values before t are exact on this grid
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j) {
-            uint32_t i = tid * kEPT + j;
-            if (i >= pos && i < t && out) stage[tid * kPad + j] = double(Ci[j]) * G;
-            if (t < cnt && i >= pos && i + 1 == t) s_c = double(Ci[j]) * G;   // c_{t-1}
-            if (t == cnt && i + 1 == cnt) s_c = double(Ci[j]) * G;
-        }
-        if (tid == 0 && t == pos) s_c = c;                           // no element on this grid
-        __syncthreads();
-        if (t >= cnt) { c = s_c; __syncthreads(); break; }
-        // step t with a real FP64 addition (the reference's own rounding)
-        if (tid == t / kEPT) {
-            double prev = s_c;
-            // element t from the staging buffer: slots >= t are still the
-            // probabilities (indexing p[] here would put it in local memory)
-            const double pt = stage[stage_slot(t)];
-            double ct = __dadd_rn(prev, pt);
-            if (out) stage[stage_slot(t)] = ct;
-            s_c = ct;
+        // slots >= t are still the probabilities
+        pos = min(cnt, t + kRun);
+        if (tid == 0 && t < cnt) {
+            double cc = s_c;
+            for (uint32_t i = t; i < pos; ++i) {
+                cc = __dadd_rn(cc, stage[stage_slot(i)]);
+                if (out) stage[stage_slot(i)] = cc;
+            }
+            s_c = cc;
         }
         __syncthreads();
         c = s_c;
-        pos = t + 1;
+        seq = false;
         __syncthreads();
     }
     if (out) {
@@ -753,16 +784,14 @@ __device__ __forceinline__ Summ block_summ(double (&p)[kEPT], int32_t gs, uint64
 #pragma unroll
                 for (int j = 0; j < kEPT; ++j) stage[stage_slot(j * kBT + threadIdx.x)] = p[j];
                 __syncthreads();
-#pragma unroll
-                for (int j = 0; j < kEPT; ++j) p[j] = stage[threadIdx.x * kPad + j];
                 staged = true;
             }
             const Grid g = grid_of(e + k);
             uint64_t t0 = 0, t1 = 0;
-#pragma unroll
-            for (int j = 0; j < kEPT; ++j) {
+#pragma unroll 1
+            for (int j = 0; j < kEPT; ++j) {   // rolled: the maps unrolled are mostly instruction fetch
                 uint64_t a0, a1, r0, r1;
-                elem_map_g(p[j], g, a0, a1);
+                elem_map_g(stage[threadIdx.x * kPad + j], g, a0, a1);
                 compose(t0, t1, a0, a1, r0, r1);
                 t0 = r0;
                 t1 = r1;
