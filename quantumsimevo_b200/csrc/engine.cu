@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <map>
 
 #include "jit.h"
@@ -38,17 +39,21 @@ uint64_t physical_to_logical_index(const qse_state* st, uint64_t P)
 }
 
 // ---- plan cache ----
-// An execute of a program that ran before on a state in the same layout (a
-// sampling loop that runs one circuit from |0..0> again and again, a repeated
-// adjoint sweep at fixed parameters) reuses that plan: its pass programs, its
-// kernels' sources and the compiled kernels.  Planning a 500-gate circuit and
-// generating its kernels' sources takes close to a millisecond of host time,
-// during which the device has nothing queued.  An entry's key holds every input
-// the plan depends on, written field by field (plan::Gate has padding).
+// An execute of a program whose gates ran before on a state in the same layout
+// (a sampling loop that runs one circuit from |0..0> again and again, an
+// optimiser that runs it with new angles at every step) reuses that plan: its
+// pass programs, its kernels' sources and the compiled kernels, with its numbers
+// set to the new angles and matrices.  Planning a gradient of a 1056-gate QAOA
+// circuit and generating its kernels' sources takes 9 ms of host time, during
+// which the device has nothing queued; setting its numbers takes 0.1 ms.  An
+// entry's key holds every input that the plan and the sources depend on besides
+// those numbers, written field by field (plan::Gate has padding).
 struct PlanEntry {
     std::string key;
     size_t hash = 0;
     uint64_t used = 0;
+    plan::Options opt;                              // as planned
+    std::vector<double> numbers;                    // angles and matrices that pl and srcs hold
     plan::Plan pl;
     bool use_jit = false;
     std::vector<jit::Source> srcs;
@@ -82,13 +87,13 @@ struct KeyWriter {
         put(o.k); put(o.rb); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
         put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.keep_gphase);
     }
+    // everything but the angles and the matrices
     void put_gates(const std::vector<plan::Gate>& gates)
     {
         put(uint64_t(gates.size()));
-        s.reserve(s.size() + gates.size() * 96);
+        s.reserve(s.size() + gates.size() * 24);
         for (const plan::Gate& g : gates) {
-            put(g.type); put(g.t); put(g.c); put(g.cmask); put(g.theta); put(g.grad);
-            s.append(reinterpret_cast<const char*>(g.m), sizeof g.m);
+            put(g.type); put(g.t); put(g.c); put(g.cmask); put(g.grad);
         }
     }
     // the state's layout: qubit count and logical -> physical map
@@ -98,6 +103,18 @@ struct KeyWriter {
         s.append(reinterpret_cast<const char*>(st->perm), st->n * sizeof(uint32_t));
     }
 };
+
+// The angles of gates (and the elements of the 2x2 ones), in order.
+std::vector<double> gate_numbers(const std::vector<plan::Gate>& gates)
+{
+    std::vector<double> v;
+    v.reserve(gates.size());
+    for (const plan::Gate& g : gates) {
+        v.push_back(g.theta);
+        if (g.type == QSE_GATE_2X2) v.insert(v.end(), g.m, g.m + 8);
+    }
+    return v;
+}
 
 std::shared_ptr<PlanEntry> plan_cache_find(qse_ctx* ctx, const std::string& key, size_t hash)
 {
@@ -335,7 +352,7 @@ constexpr size_t kJitMaxNewKernels = 32;
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
 // compiling, for the interpreter (angle accumulators, use_jit = false).
-// Specialised plans are kept in the context's plan cache.
+// Plans are kept in the context's plan cache.
 std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>& gates, plan::Options opt, int ns,
                                     bool prob_out = false)
 {
@@ -343,49 +360,58 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     auto e = std::make_shared<PlanEntry>();
     e->use_jit = ctx->jit != 0;
     opt.acc_mul = e->use_jit;
-    if (e->use_jit) {
-        KeyWriter w;
-        w.put('F');
-        w.put(ctx->jit);
-        w.put(ns);
-        w.put(prob_out);
-        w.put(st->lazy_basis);
-        w.put(st->lazy_basis ? st->lazy_umask : 0);
-        w.put(st->lazy_basis ? st->lazy_pmask : 0);
-        const char* dbg = std::getenv("QSE_DEBUG_BOUNDS");   // read by jit::generate
-        w.s.append(dbg ? dbg : "");
-        w.put('\0');
-        w.put_options(opt);
-        w.put_state(st);
-        w.put_gates(gates);
-        e->key = std::move(w.s);
-        e->hash = std::hash<std::string>{}(e->key);
-        if (auto hit = plan_cache_find(ctx, e->key, e->hash)) return hit;
+    KeyWriter w;
+    w.put('F');
+    w.put(ctx->jit);
+    w.put(ns);
+    w.put(prob_out);
+    w.put(st->lazy_basis);
+    w.put(st->lazy_basis ? st->lazy_umask : 0);
+    w.put(st->lazy_basis ? st->lazy_pmask : 0);
+    const char* dbg = std::getenv("QSE_DEBUG_BOUNDS");   // read by jit::generate
+    w.s.append(dbg ? dbg : "");
+    w.put('\0');
+    w.put_options(opt);
+    w.put_state(st);
+    w.put_gates(gates);
+    e->key = std::move(w.s);
+    e->hash = std::hash<std::string>{}(e->key);
+    std::vector<double> numbers = gate_numbers(gates);
+    if (auto hit = plan_cache_find(ctx, e->key, e->hash)) {
+        if (hit->numbers.size() != numbers.size() ||
+            std::memcmp(hit->numbers.data(), numbers.data(), numbers.size() * sizeof(double)) != 0) {
+            plan::bind_angles(hit->pl, gates, hit->opt);
+            for (size_t i = 0; i < hit->srcs.size(); ++i) jit::bind_params(hit->srcs[i], hit->pl.passes[i]);
+            hit->numbers = std::move(numbers);
+        }
+        return hit;
     }
+    e->numbers = std::move(numbers);
+    e->opt = opt;
     e->pl = plan::build(gates, st->n, st->perm, opt);
-    if (!e->use_jit) return e;
     const plan::Plan& pl = e->pl;
-    e->srcs.reserve(pl.passes.size());
-    // the last pass may also write the probabilities in logical order
-    uint8_t lpos[64] = {0};
-    for (uint32_t q = 0; q < st->n; ++q) lpos[pl.perm_final[q]] = uint8_t(q);
-    for (size_t i = 0; i < pl.passes.size(); ++i) {
-        const bool basis_in = i == 0 && ns == 1 && st->lazy_basis;
-        const bool prob = prob_out && ns == 1 && i + 1 == pl.passes.size();
-        e->srcs.push_back(jit::generate(pl.passes[i], ns, basis_in, ctx->jit == 2, st->n >= jit::kPreGroupQubits,
-                                        basis_in ? st->lazy_umask : 0, prob ? lpos : nullptr,
-                                        basis_in ? st->lazy_pmask : 0));
+    if (e->use_jit) {
+        e->srcs.reserve(pl.passes.size());
+        // the last pass may also write the probabilities in logical order
+        uint8_t lpos[64] = {0};
+        for (uint32_t q = 0; q < st->n; ++q) lpos[pl.perm_final[q]] = uint8_t(q);
+        for (size_t i = 0; i < pl.passes.size(); ++i) {
+            const bool basis_in = i == 0 && ns == 1 && st->lazy_basis;
+            const bool prob = prob_out && ns == 1 && i + 1 == pl.passes.size();
+            e->srcs.push_back(jit::generate(pl.passes[i], ns, basis_in, ctx->jit == 2, st->n >= jit::kPreGroupQubits,
+                                            basis_in ? st->lazy_umask : 0, prob ? lpos : nullptr,
+                                            basis_in ? st->lazy_pmask : 0));
+        }
+        if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > kJitMaxNewKernels) {
+            e->use_jit = false;
+            e->srcs.clear();
+            opt.acc_mul = false;
+            opt.rb = std::min(opt.rb, 4u);   // the interpreter kernel holds at most 16 amplitudes per thread
+            e->opt = opt;
+            e->pl = plan::build(gates, st->n, st->perm, opt);
+        }
     }
-    if (st->n >= kJitAlwaysQubits || jit::count_uncached(e->srcs) <= kJitMaxNewKernels) {
-        plan_cache_insert(ctx, e);
-        return e;
-    }
-    e->use_jit = false;
-    e->srcs.clear();
-    e->key.clear();
-    opt.acc_mul = false;
-    opt.rb = std::min(opt.rb, 4u);   // the interpreter kernel holds at most 16 amplitudes per thread
-    e->pl = plan::build(gates, st->n, st->perm, opt);
+    plan_cache_insert(ctx, e);
     return e;
 }
 

@@ -220,10 +220,18 @@ struct Gen {
         return s;
     }
 
+    std::vector<Source::PrmRef> refs;
+    std::vector<uint32_t> const_ops;
     uint32_t push(double v)
     {
         prm.push_back(v);
         return uint32_t(prm.size() - 1);
+    }
+    // a parameter that is op's a or b
+    uint32_t push_op(const plan::KOp& op, Source::PrmRef::Kind k)
+    {
+        refs.push_back({k, uint32_t(prm.size()), uint32_t(&op - P.ops.data()), 0});
+        return push(k == Source::PrmRef::op_a ? op.a : op.b);
     }
 
     std::string cond(uint16_t tcond, uint64_t ocond) const
@@ -287,11 +295,11 @@ struct Gen {
     // over the 32 lanes, built once in the prologue; groups conditioned on
     // warp bits stay per-thread multiplies (uniform within a warp).
     struct Item { uint16_t tcond; uint16_t g; };
-    struct Fac { std::vector<Item> items; bool hc = false; double ca = 1.0, cb = 0.0; };
+    struct Fac { std::vector<Item> items; std::vector<uint32_t> consts; };   // consts: K_FLUSH_ALL ops
     static constexpr uint32_t kMaxTables = 32;
     static constexpr int kThrChain = 5;   // chain index of the thread accumulator (after ar0..ar4)
     uint32_t max_tables = kMaxTables;   // 0 with precomputed group values (no prologue)
-    std::vector<plan::KOp> run_ops;
+    std::vector<uint32_t> run_ops;   // indices into P.ops
     std::vector<Item> chain[kThrChain + 1];   // pending accumulator groups: ar0..ar4, at
     std::ostringstream tabs;      // prologue code building the lane tables
     uint32_t ntab = 0;
@@ -306,7 +314,7 @@ struct Gen {
     void emit_op(const plan::KOp& op)
     {
         if (P.acc_mul) {
-            if (diag_kind(op.kind)) { run_ops.push_back(op); return; }
+            if (diag_kind(op.kind)) { run_ops.push_back(uint32_t(&op - P.ops.data())); return; }
             // A phase generator's gradient sums sign * Im(conj(l) s) per
             // amplitude, which the diagonal phases still pending for both
             // states leave unchanged (unless a pending constant is not of unit
@@ -330,8 +338,8 @@ struct Gen {
     // no pending constant of the open run scales the amplitudes
     bool run_unimodular() const
     {
-        for (const plan::KOp& k : run_ops)
-            if (k.kind == plan::K_FLUSH_ALL && std::fabs(k.a * k.a + k.b * k.b - 1.0) > 1e-12) return false;
+        for (uint32_t i : run_ops)
+            if (P.ops[i].kind == plan::K_FLUSH_ALL && P.ops[i].q == 2) return false;
         return true;
     }
 
@@ -346,15 +354,18 @@ struct Gen {
         for (const Item& it : F.items) ((it.tcond & ~31u) == 0 ? L : W).push_back(it);
         const std::string v = "f" + std::to_string(nvar++);
         std::string cst;
-        if (F.hc) {
-            const uint32_t ci = push(F.ca);
-            push(F.cb);
+        const bool hc = !F.consts.empty();
+        if (hc) {
+            const uint32_t ci = push(1.0);
+            push(0.0);
+            refs.push_back({Source::PrmRef::constant, ci, uint32_t(const_ops.size()), uint32_t(F.consts.size())});
+            const_ops.insert(const_ops.end(), F.consts.begin(), F.consts.end());
             cst = "make_double2(P.v[" + std::to_string(ci) + "], P.v[" + std::to_string(ci + 1) + "])";
         }
-        if (ntab < max_tables && (L.size() >= 2 || (L.size() == 1 && F.hc))) {
+        if (ntab < max_tables && (L.size() >= 2 || (L.size() == 1 && hc))) {
             const uint32_t t = ntab++;
             tabs << "  if ((tid >> 5) == " << (t % NW) << "u) { const u32 l = tid & 31u; double2 v = "
-                 << (F.hc ? cst : std::string("make_double2(1.0, 0.0)")) << ";";
+                 << (hc ? cst : std::string("make_double2(1.0, 0.0)")) << ";";
             for (const Item& it : L) {
                 if (it.tcond) tabs << " if (" << cond_t("l", it.tcond) << ")";
                 tabs << " v = cmul(v, gv[" << it.g << "]);";
@@ -364,7 +375,7 @@ struct Gen {
         } else {
             size_t i = 0;
             o << "    double2 " << v << " = ";
-            if (F.hc) o << cst;
+            if (hc) o << cst;
             else if (!L.empty()) {
                 const Item& it = L[i++];
                 if (it.tcond) o << cond_t("tid", it.tcond) << " ? gv[" << it.g << "] : make_double2(1.0, 0.0)";
@@ -392,7 +403,8 @@ struct Gen {
             d.insert(d.end(), chain[c].begin(), chain[c].end());
             chain[c].clear();
         };
-        for (const KOp& op : run_ops) {
+        for (uint32_t oi : run_ops) {
+            const KOp& op = P.ops[oi];
             switch (op.kind) {
             case K_ACC_REG: chain[op.p].push_back(Item{op.tcond, op.g}); break;
             case K_ACC_THR: chain[kThrChain].push_back(Item{op.tcond, op.g}); break;
@@ -402,13 +414,7 @@ struct Gen {
                 for (uint32_t r = 0; r < P.rb; ++r)
                     if ((op.f >> r) & 1) take(int(r), 1 << r);
                 take(kThrChain, 0);
-                if (!(op.a == 1.0 && op.b == 0.0)) {
-                    Fac& f = fac[0];
-                    const double a = f.ca * op.a - f.cb * op.b, b = f.ca * op.b + f.cb * op.a;
-                    f.ca = a;
-                    f.cb = b;
-                    f.hc = true;
-                }
+                if (op.q) fac[0].consts.push_back(oi);
                 break;
             }
             default: break;
@@ -416,7 +422,7 @@ struct Gen {
         }
         run_ops.clear();
         for (auto it = fac.begin(); it != fac.end();)
-            it = (it->second.items.empty() && !it->second.hc) ? fac.erase(it) : std::next(it);
+            it = (it->second.items.empty() && it->second.consts.empty()) ? fac.erase(it) : std::next(it);
         if (fac.empty()) return;
         qv = false;   // the phases change the registers
         o << "  {\n";
@@ -1015,15 +1021,18 @@ struct Gen {
         case K_X: guarded("opX<" + std::to_string(p) + ", " + std::to_string(op.f) + ">(@A);"); break;
         case K_Y: guarded("opY<" + std::to_string(p) + ", " + std::to_string(op.f) + ">(@A);"); break;
         case K_RX: case K_RY: {
-            uint32_t i = push(op.a);
-            push(op.b);
+            uint32_t i = push_op(op, Source::PrmRef::op_a);
+            push_op(op, Source::PrmRef::op_b);
             each_state(std::string(op.kind == K_RX ? "opRX<" : "opRY<") + std::to_string(p) + ">(@A, P.v[" +
                        std::to_string(i) + "], P.v[" + std::to_string(i + 1) + "]);");
             break;
         }
         case K_U: {
             uint32_t i = uint32_t(prm.size());
-            for (int t = 0; t < 8; ++t) push(P.mats[8 * op.g + t]);
+            for (uint32_t t = 0; t < 8; ++t) {
+                refs.push_back({Source::PrmRef::mat, uint32_t(prm.size()), 8u * op.g + t, 0});
+                push(P.mats[8 * op.g + t]);
+            }
             guarded("opU<" + std::to_string(p) + ", " + std::to_string(op.f) + ">(@A, &P.v[" + std::to_string(i) + "]);");
             break;
         }
@@ -1048,21 +1057,21 @@ struct Gen {
         case K_FLUSH_ALL: {
             for (uint32_t r = 0; r < P.rb; ++r)
                 if ((op.f >> r) & 1) emit_flush_reg(int(r));
-            const bool unit = op.a == 1.0 && op.b == 0.0;
+            const bool unit = op.q == 0;
             if (P.acc_mul) {
                 if (unit) {
                     o << "  if (notOne(at)) { const double2 e = at; at = make_double2(1.0, 0.0);";
                 } else {
-                    uint32_t i = push(op.a);
-                    push(op.b);
+                    uint32_t i = push_op(op, Source::PrmRef::op_a);
+                    push_op(op, Source::PrmRef::op_b);
                     o << "  { const double2 e = cmul(make_double2(P.v[" << i << "], P.v[" << i + 1
                       << "]), at); at = make_double2(1.0, 0.0);";
                 }
             } else if (unit) {
                 o << "  if (at != 0.0) { const double2 e = expi(at); at = 0.0;";
             } else {
-                uint32_t i = push(op.a);
-                push(op.b);
+                uint32_t i = push_op(op, Source::PrmRef::op_a);
+                push_op(op, Source::PrmRef::op_b);
                 o << "  { double2 e = make_double2(P.v[" << i << "], P.v[" << i + 1 << "]);"
                   << " if (at != 0.0) { e = cmul(e, expi(at)); at = 0.0; }";
             }
@@ -1119,7 +1128,7 @@ struct Gen {
                        (cached ? ">(qz)" : ">(a0, a1)");
                 if (!c.empty()) expr = "((" + c + ") ? " + expr + " : 0.0)";
             }
-            const uint32_t si = push(op.a);
+            const uint32_t si = push_op(op, Source::PrmRef::op_a);
             // the first kRegSlots slots of a pass accumulate in registers (one
             // warp reduction per slot at the end of the pass instead of one per
             // gate occurrence); further slots reduce immediately
@@ -1200,6 +1209,9 @@ Source generate(const plan::PassProgram& p, int nstates, bool basis_input, bool 
         s.code = g.run_streamed();
         if (g.streamed_smem() <= kStreamedSmemMax) {
             s.prm = std::move(g.prm);
+            s.refs = std::move(g.refs);
+            s.const_ops = std::move(g.const_ops);
+            bind_params(s, p);
             s.threads = 2 * g.T;
             s.smem = g.streamed_smem();
             s.streamed = true;
@@ -1215,6 +1227,9 @@ Source generate(const plan::PassProgram& p, int nstates, bool basis_input, bool 
     Source s;
     s.code = g.run();
     s.prm = std::move(g.prm);
+    s.refs = std::move(g.refs);
+    s.const_ops = std::move(g.const_ops);
+    bind_params(s, p);
     s.basis_slot = g.basis_slot;
     s.pre_gv = g.pre_gv;
     s.gv_lo = g.gv_lo;
@@ -1226,6 +1241,29 @@ Source generate(const plan::PassProgram& p, int nstates, bool basis_input, bool 
     s.smem = (size_t(1) << p.k) * 16 + p.groups.size() * 16 + size_t(g.ntab) * 32 * 16 +
              (nstates == 2 ? p.slot_src.size() * g.NW * 8 : 0) + (g.preg ? size_t(g.R) * 16 : 0);
     return s;
+}
+
+void bind_params(Source& s, const plan::PassProgram& p)
+{
+    for (const Source::PrmRef& r : s.refs) {
+        switch (r.kind) {
+        case Source::PrmRef::op_a: s.prm[r.slot] = p.ops[r.index].a; break;
+        case Source::PrmRef::op_b: s.prm[r.slot] = p.ops[r.index].b; break;
+        case Source::PrmRef::mat: s.prm[r.slot] = p.mats[r.index]; break;
+        case Source::PrmRef::constant: {
+            double a = 1.0, b = 0.0;
+            for (uint32_t i = 0; i < r.count; ++i) {
+                const plan::KOp& op = p.ops[s.const_ops[r.index + i]];
+                const double x = a * op.a - b * op.b, y = a * op.b + b * op.a;
+                a = x;
+                b = y;
+            }
+            s.prm[r.slot] = a;
+            s.prm[r.slot + 1] = b;
+            break;
+        }
+        }
+    }
 }
 
 size_t count_uncached(const std::vector<Source>& srcs)

@@ -20,6 +20,15 @@ struct Source {
     bool prob = false;               // writes the probability side output (prob_lpos)
     bool prob_bsum = false;          // ... with its 4096-block sums
     std::vector<double> prm;  // the kernel's parameter block (angles, matrices, scales)
+    // where the numbers in prm come from (bind_params); the code holds none of them
+    struct PrmRef {
+        enum Kind : uint8_t { op_a, op_b, mat, constant } kind;
+        uint32_t slot;
+        uint32_t index;       // op, element of mats, or first entry of const_ops
+        uint32_t count;       // constant: its K_FLUSH_ALL ops, multiplied in order into slot, slot + 1
+    };
+    std::vector<PrmRef> refs;
+    std::vector<uint32_t> const_ops;
     uint32_t threads = 0;
     size_t smem = 0;
     int basis_slot = -1;      // basis-input passes: the prm slot that takes the basis index
@@ -75,6 +84,9 @@ size_t compile_only(const Source& s);
 Source generate(const plan::PassProgram& p, int nstates, bool basis_input = false, bool streamed = false,
                 bool precomputed_groups = false, uint64_t compact_mask = 0, const uint8_t* prob_lpos = nullptr,
                 uint64_t product_mask = 0);
+// sets s.prm to the numbers of p, the program s was generated from with other
+// angles (plan::bind_angles)
+void bind_params(Source& s, const plan::PassProgram& p);
 // distinct sources among srcs that are not compiled yet
 size_t count_uncached(const std::vector<Source>& srcs);
 // compiled kernels for every source (cached by source text; missing ones are compiled in parallel)

@@ -102,6 +102,13 @@ struct Absorbed {
     uint64_t psup;   // physical support (diagonal)
 };
 
+// What the passes of a plan have deferred: the scale of their unscaled
+// Hadamards, and whether RZ's global phase is part of it.
+struct Carry {
+    double scale = 1.0;
+    bool phased = false;
+};
+
 // ---------- lowering of one pass ----------
 class Lowering {
 public:
@@ -118,12 +125,12 @@ public:
     // the current register bits; only when none is left does the pass change
     // register layout, to the bits with the most ready gates.  For the QFT
     // this halves the layouts of program order (one per block of register bits).
-    // carry: constant factor deferred by the previous passes of the plan
+    // carry: the constant factor deferred by the previous passes of the plan
     // (the unscaled Hadamards' 1/sqrt2 and RZ's global phase); the pass
     // applies carry times its own factor when it is the last pass (apply),
-    // else it applies nothing and returns the product for the next pass
-    std::pair<double, double> run(const std::vector<Absorbed>& abs, double gphase, std::pair<double, double> carry,
-                                  bool apply)
+    // else it applies nothing and returns the product for the next pass.  Only
+    // what the factor is made of is decided here, its value in bind_angles
+    Carry run(const std::vector<Absorbed>& abs, const Carry& carry, bool apply)
     {
         const int m = int(abs.size());
         std::vector<std::vector<int>> succ(m);
@@ -229,7 +236,7 @@ public:
                     if (reg_pos(loc_[abs[i].pt]) >= 0) { pick = i; break; }
                 if (pick < 0) {
                     if (ready_n.empty()) fail(QSE_ERR_INVALID, "internal: pass schedule stalled");
-                    close_all(false, 1.0, 0.0);
+                    close_all(-1, 0);
                     std::vector<int> prev(reg_, reg_ + P.rb);
                     pick_regs(prev.data());
                     KOp t{};
@@ -251,7 +258,7 @@ public:
             const Gate& g = *a.g;
             if (a.cls == C_DIAG) {
                 if (opt_.grads && g.grad >= 0) emit_grad_diag(a);
-                add_diag_terms(a, gphase);
+                add_diag_terms(a);
                 continue;
             }
             const int p = reg_pos(loc_[a.pt]);
@@ -264,19 +271,22 @@ public:
                 set_control(op, a.pc);
             } else {
                 switch (g.type) {
-                case QSE_GATE_H: op.kind = K_H; scale_ *= kInvSqrt2; break;
+                case QSE_GATE_H:
+                    op.kind = K_H;
+                    scale_ *= kInvSqrt2;
+                    event(PassProgram::ScaleEvent::hadamard, 0);
+                    break;
                 case QSE_GATE_X: op.kind = K_X; break;
                 case QSE_GATE_Y: op.kind = K_Y; break;
                 case QSE_GATE_RX: case QSE_GATE_RY:
                     op.kind = g.type == QSE_GATE_RX ? K_RX : K_RY;
-                    op.a = std::cos(g.theta / 2.0);
-                    op.b = std::sin(g.theta / 2.0);
                     P.op_angles.push_back(AngleRef{uint32_t(P.ops.size()), uint32_t(a.src)});
                     break;
                 case QSE_GATE_2X2:
                     op.kind = K_U;
                     op.g = uint16_t(P.mats.size() / 8);
                     P.mats.insert(P.mats.end(), g.m, g.m + 8);
+                    P.mat_src.push_back(uint32_t(a.src));
                     break;
                 default: fail(QSE_ERR_UNSUPPORTED, "internal: unexpected non-diagonal type");
                 }
@@ -286,21 +296,16 @@ public:
             // each unscaled Hadamard grows the stored values by sqrt2: apply the
             // pending 1/sqrt2 factors before they fall below kFlushScale
             if (scale_ < kFlushScale) {
-                close_all(true, scale_, 0.0);
+                close_all(PassProgram::ScaleEvent::flush, 2);
                 scale_ = 1.0;
             }
         }
-        const double ga = opt_.keep_gphase ? scale_ * std::cos(gphase_) : scale_;
-        const double gb = opt_.keep_gphase ? scale_ * std::sin(gphase_) : 0.0;
-        const std::pair<double, double> c{carry.first * ga - carry.second * gb, carry.first * gb + carry.second * ga};
+        const Carry c{carry.scale * scale_, carry.phased || (opt_.keep_gphase && !P.gphase_src.empty())};
         // the deferred constant stays above kFlushScale in magnitude, so the
         // stored amplitudes stay below 1 / kFlushScale times their true size
-        if (apply || std::hypot(c.first, c.second) < kFlushScale) {
-            close_all(true, c.first, c.second);
-            return {1.0, 0.0};
-        }
-        close_all(true, 1.0, 0.0);
-        return c;
+        P.deferred = !apply && c.scale >= kFlushScale;
+        close_all(PassProgram::ScaleEvent::last, P.deferred ? 0 : c.scale != 1.0 ? 2 : c.phased ? 1 : 0);
+        return P.deferred ? c : Carry{};
     }
 
 private:
@@ -311,8 +316,9 @@ private:
     int reg_[5] = {0, 0, 0, 0, 0};
     int thr_[16];
     int nthr_ = 0;
-    double gphase_ = 0.0;
     double scale_ = 1.0;   // product of the 1/sqrt2 factors of the unscaled K_H applied so far
+
+    void event(PassProgram::ScaleEvent::Kind kind, size_t op) { P.scale_events.push_back({kind, uint32_t(op)}); }
 
     struct OG {
         uint8_t kind, p, f;
@@ -413,7 +419,7 @@ private:
 
     void add_term(uint64_t sup, double theta, int32_t src)
     {
-        if (sup == 0) { gphase_ += theta; return; }
+        if (sup == 0) fail(QSE_ERR_INVALID, "internal: diagonal gate without qubits");
         uint8_t f;
         uint16_t tc;
         uint64_t oc;
@@ -436,7 +442,7 @@ private:
         it->second.src.push_back(src);
     }
 
-    void add_diag_terms(const Absorbed& a, double& /*unused*/)
+    void add_diag_terms(const Absorbed& a)
     {
         const Gate& g = *a.g;
         switch (g.type) {
@@ -444,7 +450,7 @@ private:
         case QSE_GATE_PHASE: case QSE_GATE_CPHASE: case QSE_GATE_MCPHASE: add_term(a.psup, g.theta, int32_t(a.src)); break;
         case QSE_GATE_RZ:  // diag(e^{-it/2}, e^{it/2}) = e^{-it/2} diag(1, e^{it})
             add_term(a.psup, g.theta, int32_t(a.src));
-            gphase_ += -g.theta / 2.0;
+            P.gphase_src.push_back(uint32_t(a.src));
             break;
         default: fail(QSE_ERR_UNSUPPORTED, "internal: unexpected diagonal type");
         }
@@ -488,7 +494,9 @@ private:
         }
     }
 
-    void close_all(bool final, double ca, double cb)
+    // kind: the scale event of a flush that takes the pass constant (q: its
+    // kind, as in K_FLUSH_ALL), or -1 for a change of layout
+    void close_all(int kind, uint8_t q)
     {
         uint8_t fmask = 0;
         bool thr = false;
@@ -505,12 +513,13 @@ private:
             if (og.kind == K_ACC_THR) thr = true;
         }
         open_.clear();
-        if (final || fmask || thr) {
+        if (kind >= 0 || fmask || thr) {
             KOp fl{};
             fl.kind = K_FLUSH_ALL;
             fl.f = fmask;
-            fl.a = final ? ca : 1.0;
-            fl.b = final ? cb : 0.0;
+            fl.q = q;
+            fl.a = 1.0;
+            if (kind >= 0) event(PassProgram::ScaleEvent::Kind(kind), P.ops.size());
             P.ops.push_back(fl);
         }
     }
@@ -535,7 +544,7 @@ private:
         else if (g.type == QSE_GATE_RY) op.kind = K_GRAD_Y;
         else return;
         op.g = new_slot(g.grad);
-        op.a = scale_ * scale_;   // both states still lack the pass's pending H scale
+        event(PassProgram::ScaleEvent::gradient, P.ops.size());   // both states still lack the pass's pending scale
         P.ops.push_back(op);
     }
 
@@ -555,10 +564,47 @@ private:
             return;
         }
         op.g = new_slot(g.grad);
-        op.a = scale_ * scale_;   // both states still lack the pass's pending H scale
+        event(PassProgram::ScaleEvent::gradient, P.ops.size());
         P.ops.push_back(op);
     }
 };
+
+void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
+{
+    double cr = 1.0, ci = 0.0;   // the constant deferred by the passes so far
+    for (PassProgram& P : plan.passes) {
+        for (const AngleRef& r : P.op_angles) {
+            P.ops[r.index].a = std::cos(gates[r.src].theta / 2.0);
+            P.ops[r.index].b = std::sin(gates[r.src].theta / 2.0);
+        }
+        for (const AngleRef& r : P.term_angles) P.terms[r.index].theta = gates[r.src].theta;
+        for (size_t i = 0; i < P.mat_src.size(); ++i) std::copy(gates[P.mat_src[i]].m, gates[P.mat_src[i]].m + 8, &P.mats[8 * i]);
+        double gphase = 0.0, scale = 1.0;
+        for (uint32_t s : P.gphase_src) gphase += -gates[s].theta / 2.0;
+        for (const PassProgram::ScaleEvent& e : P.scale_events) {
+            switch (e.kind) {
+            case PassProgram::ScaleEvent::hadamard: scale *= kInvSqrt2; break;
+            case PassProgram::ScaleEvent::gradient: P.ops[e.op].a = scale * scale; break;
+            case PassProgram::ScaleEvent::flush:
+                P.ops[e.op].a = scale;
+                scale = 1.0;
+                break;
+            case PassProgram::ScaleEvent::last: {
+                const double ga = opt.keep_gphase ? scale * std::cos(gphase) : scale;
+                const double gb = opt.keep_gphase ? scale * std::sin(gphase) : 0.0;
+                const double r = cr * ga - ci * gb, i = cr * gb + ci * ga;
+                cr = P.deferred ? r : 1.0;
+                ci = P.deferred ? i : 0.0;
+                if (!P.deferred) {
+                    P.ops[e.op].a = r;
+                    P.ops[e.op].b = i;
+                }
+                break;
+            }
+            }
+        }
+    }
+}
 
 }  // namespace
 
@@ -617,7 +663,7 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
     // forward plans defer every pass's constant factor to the last pass (no
     // caller reads the state between the passes of one plan); gradient plans
     // scale each pass, their K_GRAD_* weights assume it
-    std::pair<double, double> carry{1.0, 0.0};
+    Carry carry;
 
     // remaining[head..) are the gates still to plan, in order
     size_t head = 0;
@@ -628,7 +674,6 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         std::vector<Absorbed> abs;
         std::vector<size_t> deferred;
         uint32_t nN = 0, nterms = 0, nslots = 0;
-        double gph = 0.0;
         const uint64_t allq = n >= 64 ? ~uint64_t(0) : (bit(n) - 1);
         size_t stop = remaining.size();   // first gate this pass did not look at
         for (size_t r = head; r < remaining.size(); ++r) {
@@ -691,7 +736,7 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         prog.ngates = uint32_t(abs.size());
         Lowering low(prog, n, opt);
         const bool last = deferred.empty() && stop == remaining.size();
-        carry = low.run(abs, gph, carry, opt.grads || last);
+        carry = low.run(abs, carry, opt.grads || last);
         plan.passes.push_back(std::move(prog));
         // next: this pass's deferred gates, then the ones it did not look at
         // (written in place just before those, no copy of the unscanned rest)
@@ -699,7 +744,14 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         std::copy(deferred.begin(), deferred.end(), remaining.begin() + std::ptrdiff_t(head));
     }
     for (uint32_t q = 0; q < 64; ++q) plan.perm_final[q] = perm[q];
+    bind_gates(plan, gates, opt);
     return plan;
+}
+
+void bind_angles(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
+{
+    std::vector<Gate> fused;
+    bind_gates(plan, (opt.zz_fuse && fuse_zz(gates, fused)) ? fused : gates, opt);
 }
 
 std::string describe(const Plan& p)

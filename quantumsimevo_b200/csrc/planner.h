@@ -32,7 +32,8 @@ enum KKind : uint8_t {
     K_ACC_REG,     // if thread cond: acc[p] += group value g   (acc_mul: acc[p] *= (cos, sin) g)
     K_PHD,         // if thread cond: amplitudes with (j & f) == f *= group (cos, sin) g
     K_FLUSH_REG,   // amplitudes with bit p *= e^{i acc[p]}; acc[p] = 0
-    K_FLUSH_ALL,   // flush acc[p] for p in f, then all amplitudes *= e^{i acc_thr} * (a + ib)
+    K_FLUSH_ALL,   // flush acc[p] for p in f, then all amplitudes *= e^{i acc_thr} * (a + ib);
+                   // q: 0 = the constant is 1, 1 = it has modulus 1, 2 = any
     K_TRANSPOSE,   // exchange through shared memory into layout g
     K_GRAD_X,      // slot g += sum_pairs Im(conj(l0) s1 + conj(l1) s0)         (RX generator)
     K_GRAD_Y,      // slot g += sum_pairs Re(conj(l1) s0) - Re(conj(l0) s1)     (RY generator)
@@ -107,6 +108,18 @@ struct PassProgram {
     std::vector<uint64_t> phys_support;
     uint32_t ngates = 0;            // source gates absorbed
     uint32_t n_nondiag = 0;
+    // How the program's numbers follow from the source gates, in emission order,
+    // besides op_angles and term_angles (bind_angles walks them): the pending
+    // scale of the unscaled Hadamards and the ops that take it, the RZ gates
+    // whose global phase the pass constant carries, and the matrices' gates.
+    struct ScaleEvent {
+        enum Kind : uint8_t { hadamard, gradient, flush, last } kind;
+        uint32_t op;                // index into ops (not for hadamard)
+    };
+    std::vector<ScaleEvent> scale_events;
+    std::vector<uint32_t> gphase_src;
+    std::vector<uint32_t> mat_src;
+    bool deferred = false;          // the pass constant goes to the next pass instead of the last flush
 };
 
 // ---- planner input ----
@@ -162,6 +175,12 @@ bool fuse_zz(const std::vector<Gate>& gates, std::vector<Gate>& out);
 // Plans gates (logical qubits) for an n-qubit state whose logical->physical
 // map is perm_in.  Throws qse::Error on invalid gates.
 Plan build(const std::vector<Gate>& gates, uint32_t n, const uint32_t* perm_in, const Options& opt);
+
+// Everything in a plan but its numbers depends on the gates' types, qubits and
+// gradient ids only: this sets the numbers (angles, matrices, constants) of a
+// plan built for gates that differ from these in theta and m at most, to what
+// build() gives for them, bit for bit.
+void bind_angles(Plan& plan, const std::vector<Gate>& gates, const Options& opt);
 
 // Planner-only debug view used by the CPU tests: for each pass, the tile
 // (physical qubits) and the source-gate indices in execution order.
