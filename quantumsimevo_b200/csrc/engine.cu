@@ -85,7 +85,7 @@ struct KeyWriter {
     void put_options(const plan::Options& o)
     {
         put(o.k); put(o.rb); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
-        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.keep_gphase);
+        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.keep_gphase);
     }
     // everything but the angles and the matrices
     void put_gates(const std::vector<plan::Gate>& gates)
@@ -359,7 +359,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     qse_ctx* ctx = st->ctx;
     auto e = std::make_shared<PlanEntry>();
     e->use_jit = ctx->jit != 0;
-    opt.acc_mul = e->use_jit;
+    opt.acc_mul = opt.unit_rot = e->use_jit;
     KeyWriter w;
     w.put('F');
     w.put(ctx->jit);
@@ -405,7 +405,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
         if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > kJitMaxNewKernels) {
             e->use_jit = false;
             e->srcs.clear();
-            opt.acc_mul = false;
+            opt.acc_mul = opt.unit_rot = false;
             opt.rb = std::min(opt.rb, 4u);   // the interpreter kernel holds at most 16 amplitudes per thread
             e->opt = opt;
             e->pl = plan::build(gates, st->n, st->perm, opt);

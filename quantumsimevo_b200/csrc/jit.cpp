@@ -1089,8 +1089,14 @@ struct Gen {
         case K_RX: case K_RY: {
             uint32_t i = push_op(op, Source::PrmRef::op_a);
             push_op(op, Source::PrmRef::op_b);
-            each_state(std::string(op.kind == K_RX ? "opRX<" : "opRY<") + std::to_string(p) + ">(@A, P.v[" +
-                       std::to_string(i) + "], P.v[" + std::to_string(i + 1) + "]);");
+            // which entry divides the matrix depends on the angle: a uniform branch
+            // on the parameter, so the same kernel serves every angle
+            const std::string r = op.kind == K_RX ? "opRX" : "opRY";
+            o << "  if (P.v[" << i + 1 << "] != 0.0) {\n";
+            each_state("  " + r + "c<" + std::to_string(p) + ">(@A, P.v[" + std::to_string(i) + "]);");
+            o << "  } else {\n";
+            each_state("  " + r + "s<" + std::to_string(p) + ">(@A, P.v[" + std::to_string(i) + "]);");
+            o << "  }\n";
             break;
         }
         case K_U: {

@@ -102,8 +102,8 @@ struct Absorbed {
     uint64_t psup;   // physical support (diagonal)
 };
 
-// What the passes of a plan have deferred: the scale of their unscaled
-// Hadamards, and whether RZ's global phase is part of it.
+// What the passes of a plan have deferred: a lower bound of the scale of their
+// unscaled Hadamards and rotations, and whether RZ's global phase is part of it.
 struct Carry {
     double scale = 1.0;
     bool phased = false;
@@ -280,6 +280,10 @@ public:
                 case QSE_GATE_Y: op.kind = K_Y; break;
                 case QSE_GATE_RX: case QSE_GATE_RY:
                     op.kind = g.type == QSE_GATE_RX ? K_RX : K_RY;
+                    if (opt_.unit_rot) {   // the divisor is at least 1/sqrt2
+                        scale_ *= kInvSqrt2;
+                        event(PassProgram::ScaleEvent::rotation, P.op_angles.size());
+                    }
                     P.op_angles.push_back(AngleRef{uint32_t(P.ops.size()), uint32_t(a.src)});
                     break;
                 case QSE_GATE_2X2:
@@ -293,8 +297,9 @@ public:
             }
             P.ops.push_back(op);
             P.n_nondiag++;
-            // each unscaled Hadamard grows the stored values by sqrt2: apply the
-            // pending 1/sqrt2 factors before they fall below kFlushScale
+            // each unscaled Hadamard grows the stored values by sqrt2, an unscaled
+            // rotation by at most that: apply the pending factors before they can
+            // fall below kFlushScale
             if (scale_ < kFlushScale) {
                 close_all(PassProgram::ScaleEvent::flush, 2);
                 scale_ = 1.0;
@@ -316,7 +321,7 @@ private:
     int reg_[5] = {0, 0, 0, 0, 0};
     int thr_[16];
     int nthr_ = 0;
-    double scale_ = 1.0;   // product of the 1/sqrt2 factors of the unscaled K_H applied so far
+    double scale_ = 1.0;   // lower bound of the pending scale: 1/sqrt2 per unscaled op applied so far
 
     void event(PassProgram::ScaleEvent::Kind kind, size_t op) { P.scale_events.push_back({kind, uint32_t(op)}); }
 
@@ -573,9 +578,13 @@ void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
 {
     double cr = 1.0, ci = 0.0;   // the constant deferred by the passes so far
     for (PassProgram& P : plan.passes) {
+        std::vector<double> divisor;
         for (const AngleRef& r : P.op_angles) {
-            P.ops[r.index].a = std::cos(gates[r.src].theta / 2.0);
-            P.ops[r.index].b = std::sin(gates[r.src].theta / 2.0);
+            const double c = std::cos(gates[r.src].theta / 2.0), s = std::sin(gates[r.src].theta / 2.0);
+            const bool by_c = std::fabs(c) >= std::fabs(s);
+            P.ops[r.index].a = !opt.unit_rot ? c : by_c ? s / c : c / s;
+            P.ops[r.index].b = !opt.unit_rot ? s : by_c ? 1.0 : 0.0;
+            divisor.push_back(by_c ? c : s);
         }
         for (const AngleRef& r : P.term_angles) P.terms[r.index].theta = gates[r.src].theta;
         for (size_t i = 0; i < P.mat_src.size(); ++i) std::copy(gates[P.mat_src[i]].m, gates[P.mat_src[i]].m + 8, &P.mats[8 * i]);
@@ -584,6 +593,7 @@ void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
         for (const PassProgram::ScaleEvent& e : P.scale_events) {
             switch (e.kind) {
             case PassProgram::ScaleEvent::hadamard: scale *= kInvSqrt2; break;
+            case PassProgram::ScaleEvent::rotation: scale *= divisor[e.op]; break;
             case PassProgram::ScaleEvent::gradient: P.ops[e.op].a = scale * scale; break;
             case PassProgram::ScaleEvent::flush:
                 P.ops[e.op].a = scale;

@@ -25,8 +25,9 @@ enum KKind : uint8_t {
     K_H,           // unscaled Hadamard on register bit p (the pass scale carries 1/sqrt2 per H)
     K_X,           // X on p, controls: register mask f, thread mask tcond, outer mask ocond
     K_Y,           // Y on p, same controls
-    K_RX,          // [[c,-is],[-is,c]] on p, (a,b) = (c,s)
-    K_RY,          // [[c,-s],[s,c]] on p
+    K_RX,          // [[c,-is],[-is,c]] on p, (a,b) = (c,s); Options::unit_rot: divided by c, (a,b) = (s/c, 1),
+                   // where |c| >= |s|, else by s, (a,b) = (c/s, 0) (the pass scale carries the divisor)
+    K_RY,          // [[c,-s],[s,c]] on p, likewise
     K_U,           // generic 2x2 on p, matrix index g, controls as K_X
     K_ACC_THR,     // if thread cond: acc_thr += group value g  (acc_mul: acc_thr *= (cos, sin) g)
     K_ACC_REG,     // if thread cond: acc[p] += group value g   (acc_mul: acc[p] *= (cos, sin) g)
@@ -110,11 +111,11 @@ struct PassProgram {
     uint32_t n_nondiag = 0;
     // How the program's numbers follow from the source gates, in emission order,
     // besides op_angles and term_angles (bind_angles walks them): the pending
-    // scale of the unscaled Hadamards and the ops that take it, the RZ gates
+    // scale of the unscaled Hadamards and rotations and the ops that take it, the RZ gates
     // whose global phase the pass constant carries, and the matrices' gates.
     struct ScaleEvent {
-        enum Kind : uint8_t { hadamard, gradient, flush, last } kind;
-        uint32_t op;                // index into ops (not for hadamard)
+        enum Kind : uint8_t { hadamard, rotation, gradient, flush, last } kind;
+        uint32_t op;                // index into ops (rotation: into op_angles; hadamard: none)
     };
     std::vector<ScaleEvent> scale_events;
     std::vector<uint32_t> gphase_src;
@@ -154,6 +155,8 @@ struct Options {
     bool zz_fuse = false;        // rewrite CNOT(c,t) RZ(th,t) CNOT(c,t) as the diagonal
                                  // RZ(th,c) PHASE(th,t) CPHASE(-2th,c,t) (same three slots;
                                  // only for plans whose angles are never rebound)
+    bool unit_rot = false;       // rotations divided by their larger entry, one FMA per component instead
+                                 // of a multiply and an FMA (kernels that take K_RX / K_RY in that form)
     bool keep_gphase = true;     // false: drop RZ's global phase (expectations and gradients
                                  // do not see it; the pass programs then depend on angles
                                  // only through op_angles / term_angles)
