@@ -763,9 +763,9 @@ struct Gen {
         src << kPrelude << "\n";
         src << "struct Prm { double v[" << std::max<size_t>(1, prm.size()) << "]; };\n";
         // resident CTAs per SM the register budget allows: 128 registers per
-        // thread, 168 for 32 amplitudes per thread (their 128 registers and the
-        // rest; three CTAs of 128 threads per SM)
-        const uint32_t budget = R >= 32 ? 168u : 128u;
+        // thread, 168 for 32 amplitudes per thread (of one state, or 16 of each of
+        // two: their 128 registers and the rest; three CTAs of 128 threads per SM)
+        const uint32_t budget = R * uint32_t(ns) >= 32 ? 168u : 128u;
         const uint32_t min_blocks = std::max(1u, std::min(8u, 65536u / (T * budget)));
         src << "extern \"C\" __global__ void __launch_bounds__(" << T << ", " << min_blocks << ") " << kernel_name() << "("
             << "double2* __restrict__ psi, double2* __restrict__ lam, const TermRec* __restrict__ terms, "
