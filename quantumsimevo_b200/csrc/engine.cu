@@ -85,7 +85,7 @@ struct KeyWriter {
     void put_options(const plan::Options& o)
     {
         put(o.k); put(o.rb); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
-        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.keep_gphase);
+        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.keep_gphase);
     }
     // everything but the angles and the matrices
     void put_gates(const std::vector<plan::Gate>& gates)
@@ -348,6 +348,13 @@ __global__ void __launch_bounds__(256) k_group_values(const plan::TermRec* __res
 // need hundreds of distinct kernels; its plan runs on the interpreter instead.
 constexpr uint32_t kJitAlwaysQubits = 22;
 constexpr size_t kJitMaxNewKernels = 32;
+// States of at least this many qubits (128 MiB, beyond the L2) plan their layouts
+// for contiguous memory accesses (Options::low_lanes), at the price of a few more
+// layout exchanges: <O> of a 28-qubit QAOA circuit 9.6 -> 7.9 ms, 25-qubit
+// random layers 1.93 -> 1.75 ms, 25-qubit layered rotations 1.18 -> 1.04 ms,
+// 26-qubit H+RZ+QFT 0.74 -> 0.75 ms.  At 22 qubits the exchanges cost more than
+// the accesses (HEA gradient 1.84 -> 1.91 ms).
+constexpr uint32_t kLowLanesQubits = 23;
 
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
@@ -548,6 +555,7 @@ plan::Options fused_options(const qse_ctx* ctx, uint32_t n)
     opt.max_gates = uint32_t(std::max(0, ctx->max_gates_per_pass));
     if (ctx->jit && (opt.max_gates == 0 || opt.max_gates > plan::kJitMaxGates)) opt.max_gates = plan::kJitMaxGates;
     opt.zz_fuse = true;
+    opt.low_lanes = n >= kLowLanesQubits;
     return opt;
 }
 
@@ -1271,6 +1279,7 @@ double adjoint(qse_state* st, const qse_op* ops, size_t nops, const double* para
     opt.grads = true;
     opt.max_terms = 512;
     opt.max_gates = plan::kJitMaxGates;
+    opt.low_lanes = st->n >= kLowLanesQubits;
     const std::shared_ptr<PlanEntry> e = plan_for(st, rev, opt, 2);
     const plan::Plan& pl = e->pl;
     Uploaded up = upload_plan(ctx, pl, e->use_jit && st->n >= jit::kPreGroupQubits);

@@ -178,13 +178,21 @@ public:
             for (int s : succ[i])
                 if (--indeg[s] == 0) make_ready(s);
         };
-        // register bits for a new layout: most ready gates, then most gates in the lookahead, then earliest
+        // register bits for a new layout: bits with ready gates, then most gates
+        // in the lookahead, then earliest.  The first and the last layout of a
+        // pass are the ones it reads and writes memory in, and a warp's accesses
+        // are contiguous where the lowest physical qubits are lane bits: with
+        // qubits 0..2 in registers each lane touches a 128-byte line of its own,
+        // and the pass stalls on the load-store unit.  With low_lanes those qubits
+        // come last in the first layout and as fill, and first once they have
+        // ready gates after it.
         auto pick_regs = [&](const int* prev) {
             std::vector<long long> score(P.k, 0);
             std::vector<int> first(P.k, 1 << 30);
+            std::vector<char> ready(P.k, 0);
             for (int i : ready_n) {
                 int b = loc_[abs[i].pt];
-                score[b] += 1000000;
+                ready[b] = 1;
                 first[b] = std::min(first[b], i);
             }
             int seen = 0;
@@ -199,6 +207,10 @@ public:
             std::vector<int> bits(P.k);
             for (uint32_t b = 0; b < P.k; ++b) bits[b] = int(b);
             std::stable_sort(bits.begin(), bits.end(), [&](int x, int y) {
+                if (ready[x] != ready[y]) return ready[x] > ready[y];
+                const bool lx = opt_.low_lanes && P.tile_phys[x] < 3, ly = opt_.low_lanes && P.tile_phys[y] < 3;
+                if (lx != ly && (!prev || !ready[x])) return ly;
+                if (lx != ly) return lx;
                 if (score[x] != score[y]) return score[x] > score[y];
                 bool px = false, py = false;
                 if (prev)

@@ -155,6 +155,7 @@ struct Options {
     bool zz_fuse = false;        // rewrite CNOT(c,t) RZ(th,t) CNOT(c,t) as the diagonal
                                  // RZ(th,c) PHASE(th,t) CPHASE(-2th,c,t) (same three slots;
                                  // only for plans whose angles are never rebound)
+    bool low_lanes = false;      // keep physical qubits 0..2 out of the registers where a pass reads and writes
     bool unit_rot = false;       // rotations divided by their larger entry, one FMA per component instead
                                  // of a multiply and an FMA (kernels that take K_RX / K_RY in that form)
     bool keep_gphase = true;     // false: drop RZ's global phase (expectations and gradients
