@@ -133,7 +133,8 @@ QSE_API const char* qse_version(void);
 QSE_API int qse_ctx_create(int device, qse_ctx** out);
 QSE_API int qse_ctx_destroy(qse_ctx* ctx);
 QSE_API int qse_ctx_synchronize(qse_ctx* ctx);
-/* fused-planner knobs: tile qubits (10..12), cap on non-diagonal gates per pass
+/* fused-planner knobs: tile qubits (10..12; 12, the default, lets states of at
+ * most 20 qubits run smaller tiles), cap on non-diagonal gates per pass
  * (0 = none; with specialised pass kernels at most 256, which bounds their
  * compile time), fusion on/off (off = one kernel per gate, the plain method). */
 QSE_API int qse_ctx_set_fusion(qse_ctx* ctx, int enabled, int tile_qubits, int max_gates_per_pass);

@@ -342,12 +342,31 @@ __global__ void __launch_bounds__(256) k_group_values(const plan::TermRec* __res
     }
 }
 
+uint32_t tile_qubits_for(const qse_ctx* ctx, uint32_t n, uint32_t rb, uint32_t kmax)
+{
+    uint32_t k = std::min<uint32_t>(std::max(ctx->tile_qubits, int(rb) + 1), kmax);
+    return std::min(k, n);
+}
+
 // Specialised pass kernels repay their compile time (NVRTC: about a second or
 // more per distinct kernel) when a pass is expensive, i.e. on large states, or
 // when few of a plan's kernels are new.  A deep circuit on a small state can
 // need hundreds of distinct kernels; its plan runs on the interpreter instead.
 constexpr uint32_t kJitAlwaysQubits = 22;
 constexpr size_t kJitMaxNewKernels = 32;
+// ... kernels with 8 amplitudes per thread (small states) compile about five times
+// faster (16-qubit layered rotations: 0.9 s for all passes instead of 4.8)
+constexpr size_t kJitMaxNewSmall = 96;
+// States of at most kSmallQubits qubits hold 8 amplitudes per thread in tiles of
+// 2^11 (up to kTile11Qubits, where more passes cost more than fuller SMs give)
+// or 2^10: with 32 per thread and 2^12 they are a few CTAs of four warps each
+// (16 at 16 qubits), bound by fetching their straight-line code, a quarter as
+// long with 8 per thread.  Layered rotations, execute and download: 12 qubits
+// 235 -> 114 us, 14 qubits 427 -> 229, 16 qubits 605 -> 348 (tiles of 2^10: 113,
+// 220, 370); on the device, 20 qubits 115 -> 93 (2^11: 105), random layers of 19
+// qubits 67 -> 63 (69).
+constexpr uint32_t kTile11Qubits = 18;
+constexpr uint32_t kSmallQubits = 20;
 // States of at least this many qubits (128 MiB, beyond the L2) plan their layouts
 // for contiguous memory accesses (Options::low_lanes), at the price of a few more
 // layout exchanges: <O> of a 28-qubit QAOA circuit 9.6 -> 7.9 ms, 25-qubit
@@ -409,11 +428,12 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
                                             basis_in ? st->lazy_umask : 0, prob ? lpos : nullptr,
                                             basis_in ? st->lazy_pmask : 0));
         }
-        if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > kJitMaxNewKernels) {
+        if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > (opt.rb <= 3 ? kJitMaxNewSmall : kJitMaxNewKernels)) {
             e->use_jit = false;
             e->srcs.clear();
             opt.acc_mul = opt.unit_rot = false;
-            opt.rb = std::min(opt.rb, ns == 2 ? 3u : 4u);   // the interpreter kernel holds at most 16 amplitudes per thread
+            opt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
+            if (ns == 1) opt.k = tile_qubits_for(ctx, st->n, 4, 12);
             e->opt = opt;
             e->pl = plan::build(gates, st->n, st->perm, opt);
         }
@@ -497,12 +517,6 @@ struct PassRunner {
     }
 };
 
-uint32_t tile_qubits_for(const qse_ctx* ctx, uint32_t n, uint32_t rb, uint32_t kmax)
-{
-    uint32_t k = std::min<uint32_t>(std::max(ctx->tile_qubits, int(rb) + 1), kmax);
-    return std::min(k, n);
-}
-
 // noisy gates of the list in program order (types in the rate map)
 void run_noise(qse_state* st, qse_noise* nz, const qse_op* ops, size_t nops, const double* inj, size_t ninj,
                qse_exec_stats* stats)
@@ -552,6 +566,10 @@ plan::Options fused_options(const qse_ctx* ctx, uint32_t n)
     // thread (128 threads, three CTAs per SM): twice the independent FP64 work
     // per thread and one layout exchange per five register qubits instead of four
     if (ctx->jit == 1 && opt.k == 12) opt.rb = 5;
+    if (ctx->jit == 1 && ctx->tile_qubits == 12 && n <= kSmallQubits) {
+        opt.k = std::min(n <= kTile11Qubits ? 11u : 10u, n);
+        opt.rb = 3;
+    }
     opt.max_gates = uint32_t(std::max(0, ctx->max_gates_per_pass));
     if (ctx->jit && (opt.max_gates == 0 || opt.max_gates > plan::kJitMaxGates)) opt.max_gates = plan::kJitMaxGates;
     opt.zz_fuse = true;

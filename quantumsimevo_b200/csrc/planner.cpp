@@ -600,8 +600,12 @@ void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
         }
         for (const AngleRef& r : P.term_angles) P.terms[r.index].theta = gates[r.src].theta;
         for (size_t i = 0; i < P.mat_src.size(); ++i) std::copy(gates[P.mat_src[i]].m, gates[P.mat_src[i]].m + 8, &P.mats[8 * i]);
-        double gphase = 0.0, scale = 1.0;
-        for (uint32_t s : P.gphase_src) gphase += -gates[s].theta / 2.0;
+        // hundreds of RZ angles add up to hundreds of radians: the sum in extended
+        // precision keeps its rounding out of the state's phase (5e-14 of it on
+        // 320 RZs in double)
+        long double gphase = 0.0L;
+        double scale = 1.0;
+        for (uint32_t s : P.gphase_src) gphase -= gates[s].theta / 2.0;
         for (const PassProgram::ScaleEvent& e : P.scale_events) {
             switch (e.kind) {
             case PassProgram::ScaleEvent::hadamard: scale *= kInvSqrt2; break;
@@ -612,8 +616,8 @@ void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
                 scale = 1.0;
                 break;
             case PassProgram::ScaleEvent::last: {
-                const double ga = opt.keep_gphase ? scale * std::cos(gphase) : scale;
-                const double gb = opt.keep_gphase ? scale * std::sin(gphase) : 0.0;
+                const double ga = opt.keep_gphase ? scale * double(std::cos(gphase)) : scale;
+                const double gb = opt.keep_gphase ? scale * double(std::sin(gphase)) : 0.0;
                 const double r = cr * ga - ci * gb, i = cr * gb + ci * ga;
                 cr = P.deferred ? r : 1.0;
                 ci = P.deferred ? i : 0.0;
