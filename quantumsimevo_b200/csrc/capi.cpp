@@ -158,8 +158,10 @@ int qse_ctx_create(int device, qse_ctx** out)
     QSE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ctx->status_host), 16, cudaHostAllocMapped));
     *reinterpret_cast<volatile unsigned*>(ctx->status_host) = 0u;
     QSE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ctx->status_dev), ctx->status_host, 0));
-    QSE_CUDA(cudaEventCreateWithFlags(&ctx->plan_event, cudaEventDisableTiming));
-    QSE_CUDA(cudaEventRecord(ctx->plan_event, ctx->stream));
+    for (cudaEvent_t* e : {&ctx->plan_event[0], &ctx->plan_event[1], &ctx->small_event}) {
+        QSE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        QSE_CUDA(cudaEventRecord(*e, ctx->stream));
+    }
     *out = ctx;
     QSE_GUARD_END
 }
@@ -176,10 +178,12 @@ int qse_ctx_destroy(qse_ctx* ctx)
     ctx->scratch.release();
     ctx->scratch2.release();
     ctx->gv_buf.release();
-    ctx->plan_host.release();
+    ctx->plan_host[0].release();
+    ctx->plan_host[1].release();
     ctx->host_small.release();
     ctx->host_small2.release();
-    if (ctx->plan_event) cudaEventDestroy(ctx->plan_event);
+    for (cudaEvent_t e : {ctx->plan_event[0], ctx->plan_event[1], ctx->small_event})
+        if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->slots)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->pass_events) cudaEventDestroy(e);

@@ -93,7 +93,9 @@ struct KeyWriter {
         put(uint64_t(gates.size()));
         s.reserve(s.size() + gates.size() * 24);
         for (const plan::Gate& g : gates) {
-            put(g.type); put(g.t); put(g.c); put(g.cmask); put(g.grad);
+            const struct { uint64_t cmask; int32_t type, grad; uint32_t t, c; } r = {g.cmask, g.type, g.grad, g.t, g.c};
+            static_assert(sizeof r == 24, "no padding in a key");
+            put(r);
         }
     }
     // the state's layout: qubit count and logical -> physical map
@@ -219,10 +221,14 @@ struct Uploaded {
     std::vector<const double2*> texp;   // per pass: (cos, sin) of each term's angle
 };
 
-// Packs every pass program into one pinned buffer and one H2D copy.  With
-// term_phases, each pass also gets the (cos, sin) of its terms' angles (for
-// k_group_values; only passes whose kernels read precomputed group values).
-Uploaded upload_plan(qse_ctx* ctx, const plan::Plan& pl, bool term_phases = false)
+// Packs every pass program into one pinned buffer and one H2D copy.  Two pinned
+// buffers take turns, so the host does not wait for the copy of the plan before
+// (a gradient's forward sweep) to come up on the stream; the device buffer is one,
+// written in stream order after the passes that read it.  The specialised kernels
+// read the terms and groups only.  With term_phases, each pass also gets the
+// (cos, sin) of its terms' angles (for k_group_values; only passes whose kernels
+// read precomputed group values).
+Uploaded upload_plan(qse_ctx* ctx, const plan::Plan& pl, bool specialised, bool term_phases)
 {
     constexpr size_t kArr = 6;
     std::vector<size_t> off(pl.passes.size() * kArr);
@@ -230,33 +236,36 @@ Uploaded upload_plan(qse_ctx* ctx, const plan::Plan& pl, bool term_phases = fals
     for (size_t i = 0; i < pl.passes.size(); ++i) {
         const plan::PassProgram& p = pl.passes[i];
         size_t* o = &off[kArr * i];
-        o[0] = total; total = align16(total + p.ops.size() * sizeof(plan::KOp));
-        o[1] = total; total = align16(total + p.layouts.size() * sizeof(plan::LayoutRec));
+        o[0] = total; total = align16(total + (specialised ? 0 : p.ops.size() * sizeof(plan::KOp)));
+        o[1] = total; total = align16(total + (specialised ? 0 : p.layouts.size() * sizeof(plan::LayoutRec)));
         o[2] = total; total = align16(total + p.terms.size() * sizeof(plan::TermRec));
         o[3] = total; total = align16(total + p.groups.size() * sizeof(plan::GroupRec));
-        o[4] = total; total = align16(total + p.mats.size() * sizeof(double));
+        o[4] = total; total = align16(total + (specialised ? 0 : p.mats.size() * sizeof(double)));
         o[5] = total; total = align16(total + (term_phases ? p.terms.size() * sizeof(double2) : 0));
     }
     total = std::max<size_t>(total, 16);
-    QSE_CUDA(cudaEventSynchronize(ctx->plan_event));
-    ctx->plan_host.reserve(total);
+    const int turn = ctx->plan_turn ^= 1;
+    QSE_CUDA(cudaEventSynchronize(ctx->plan_event[turn]));
+    ctx->plan_host[turn].reserve(total);
     ctx->plan_buf.reserve(total);
-    char* h = static_cast<char*>(ctx->plan_host.ptr);
+    char* h = static_cast<char*>(ctx->plan_host[turn].ptr);
     for (size_t i = 0; i < pl.passes.size(); ++i) {
         const plan::PassProgram& p = pl.passes[i];
         const size_t* o = &off[kArr * i];
-        std::memcpy(h + o[0], p.ops.data(), p.ops.size() * sizeof(plan::KOp));
-        std::memcpy(h + o[1], p.layouts.data(), p.layouts.size() * sizeof(plan::LayoutRec));
+        if (!specialised) {
+            std::memcpy(h + o[0], p.ops.data(), p.ops.size() * sizeof(plan::KOp));
+            std::memcpy(h + o[1], p.layouts.data(), p.layouts.size() * sizeof(plan::LayoutRec));
+            std::memcpy(h + o[4], p.mats.data(), p.mats.size() * sizeof(double));
+        }
         std::memcpy(h + o[2], p.terms.data(), p.terms.size() * sizeof(plan::TermRec));
         std::memcpy(h + o[3], p.groups.data(), p.groups.size() * sizeof(plan::GroupRec));
-        std::memcpy(h + o[4], p.mats.data(), p.mats.size() * sizeof(double));
         double2* e = reinterpret_cast<double2*>(h + o[5]);
         if (term_phases)
             for (size_t t = 0; t < p.terms.size(); ++t)
                 e[t] = make_double2(std::cos(p.terms[t].theta), std::sin(p.terms[t].theta));
     }
     QSE_CUDA(cudaMemcpyAsync(ctx->plan_buf.ptr, h, total, cudaMemcpyHostToDevice, ctx->stream));
-    QSE_CUDA(cudaEventRecord(ctx->plan_event, ctx->stream));
+    QSE_CUDA(cudaEventRecord(ctx->plan_event[turn], ctx->stream));
     char* d = static_cast<char*>(ctx->plan_buf.ptr);
     Uploaded up;
     for (size_t i = 0; i < pl.passes.size(); ++i) {
@@ -598,7 +607,7 @@ uint64_t run_fused(qse_state* st, const std::vector<plan::Gate>& gates, bool pro
         QSE_CUDA(cudaMemsetAsync(prob + st->size(), 0, (st->size() / 4096) * 8, ctx->stream));
         st->cdf_version = ~uint64_t(0);   // the buffer's cumulative values are overwritten
     }
-    Uploaded up = upload_plan(ctx, pl, use_jit && st->n >= jit::kPreGroupQubits);
+    Uploaded up = upload_plan(ctx, pl, use_jit, use_jit && st->n >= jit::kPreGroupQubits);
     PassRunner runner(st, *e, up, 1, 4);
     for (size_t i = 0; i < up.args.size(); ++i) runner.run(i, nullptr, i + 1 == up.args.size() ? prob : nullptr);
     if (!up.args.empty()) {   // the first pass wrote every amplitude
@@ -1104,23 +1113,42 @@ __global__ void __launch_bounds__(kRB, 2) k_obs(const double2* __restrict__ psi,
     }
 }
 
-// out[src[s]] = sum_b partial[s][b]
-__global__ void __launch_bounds__(kRB) k_reduce_slots(const double* __restrict__ partial, uint32_t nslots, uint64_t nb,
-                                                      const int32_t* __restrict__ src, double* __restrict__ out)
+// A gradient slot's partial sums (one per tile) of one reverse pass, added to
+// bucket src.
+struct SlotSums {
+    uint64_t off;   // first of nb doubles
+    uint32_t nb;
+    uint32_t src;
+};
+
+// out[src] += the sums of entries [seg[b], seg[b + 1]), which share src, in a
+// fixed order: one CTA per bucket and group of passes.  (A launch per pass, with
+// one dependent load after another per thread, took 18 us a pass at 24 qubits.)
+__global__ void __launch_bounds__(kRB) k_reduce_slots(const double* __restrict__ partial,
+                                                      const SlotSums* __restrict__ entries,
+                                                      const uint32_t* __restrict__ seg, double* __restrict__ out)
 {
     __shared__ double sh[kRB / 32];
-    for (uint32_t s = blockIdx.x; s < nslots; s += gridDim.x) {
-        double acc = 0.0;
-        for (uint64_t b = threadIdx.x; b < nb; b += blockDim.x) acc += partial[uint64_t(s) * nb + b];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int i = 0; i < kRB / 32; ++i) t += sh[i];
-            out[src[s]] += t;
-        }
-        __syncthreads();
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    uint32_t src = 0;
+    for (uint32_t i = seg[blockIdx.x]; i < seg[blockIdx.x + 1]; ++i) {
+        const SlotSums e = entries[i];
+        const double* p = partial + e.off;
+        src = e.src;
+        uint32_t b = threadIdx.x;
+        for (; b + 3 * kRB < e.nb; b += 4 * kRB)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] += p[b + k * kRB];
+        for (; b < e.nb; b += kRB) acc[0] += p[b];
+    }
+    double v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int i = 0; i < kRB / 32; ++i) t += sh[i];
+        out[src] += t;
     }
 }
 
@@ -1167,7 +1195,21 @@ ObsDev upload_obs(qse_state* st, const qse_observable* obs, char* dbase, char* h
     return o;
 }
 
-double run_obs(qse_state* st, const qse_observable* obs, double2* lam)
+// <O>'s partial sums on their way to host_small; valid after a synchronisation.
+struct ObsRun {
+    const double* partial;
+    unsigned count;
+    double value() const
+    {
+        double acc = 0.0;
+        for (unsigned b = 0; b < count; ++b) acc += partial[b];
+        return acc;
+    }
+};
+
+// Enqueues <psi|O|psi> (and lam = O psi if lam != nullptr).  The caller
+// synchronises before host_small is used again.
+ObsRun launch_obs(qse_state* st, const qse_observable* obs, double2* lam)
 {
     materialize(st);
     qse_ctx* ctx = st->ctx;
@@ -1176,12 +1218,13 @@ double run_obs(qse_state* st, const qse_observable* obs, double2* lam)
     const uint64_t chunks = (size + uint64_t(kRB) * kObsR - 1) / (uint64_t(kRB) * kObsR);
     const unsigned grid = unsigned(std::min<uint64_t>(chunks, uint64_t(ctx->num_sms) * 8));
     size_t obytes = align16(16 * obs->nterms);
+    QSE_CUDA(cudaEventSynchronize(ctx->small_event));   // host_small may still feed an earlier copy
     ctx->scratch.reserve(obytes + size_t(grid) * 8 + 16);
     ctx->host_small.reserve(obytes + size_t(grid) * 8 + 16);
-    QSE_CUDA(cudaStreamSynchronize(ctx->stream));  // host_small may still feed an earlier copy
     char* d = static_cast<char*>(ctx->scratch.ptr);
     char* h = static_cast<char*>(ctx->host_small.ptr);
     ObsDev o = upload_obs(st, obs, d, h);
+    QSE_CUDA(cudaEventRecord(ctx->small_event, ctx->stream));
     double* partial = reinterpret_cast<double*>(d + obytes);
     k_obs<<<grid, kRB, 16 * obs->nterms, ctx->stream>>>(reinterpret_cast<const double2*>(st->amp), lam, size, o.z, o.w,
                                                         o.nt, o.f, o.c, partial);
@@ -1189,10 +1232,7 @@ double run_obs(qse_state* st, const qse_observable* obs, double2* lam)
     count_launch(ctx);
     double* hp = reinterpret_cast<double*>(h + obytes);
     QSE_CUDA(cudaMemcpyAsync(hp, partial, size_t(grid) * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    QSE_CUDA(cudaStreamSynchronize(ctx->stream));
-    double acc = 0.0;
-    for (unsigned b = 0; b < grid; ++b) acc += hp[b];
-    return acc;
+    return ObsRun{hp, grid};
 }
 
 plan::Gate inverse_gate(const qse_op& op, double theta, int32_t grad)
@@ -1223,7 +1263,20 @@ bool parameterised(int type)
 
 }  // namespace
 
-double expectation(qse_state* st, const qse_observable* obs) { return run_obs(st, obs, nullptr); }
+double expectation(qse_state* st, const qse_observable* obs)
+{
+    const ObsRun r = launch_obs(st, obs, nullptr);
+    QSE_CUDA(cudaStreamSynchronize(st->ctx->stream));
+    return r.value();
+}
+
+namespace {
+// partial sums of the reverse passes kept before they are reduced
+constexpr size_t kMaxPartialBytes = size_t(64) << 20;
+
+double adjoint_sweep(qse_state* st, const qse_op* ops, size_t nops, const double* params, size_t nparams,
+                     const ObsRun& obs_run, double* grad);
+}  // namespace
 
 double adjoint(qse_state* st, const qse_op* ops, size_t nops, const double* params, size_t nparams,
                const qse_observable* obs, double* grad)
@@ -1234,8 +1287,20 @@ double adjoint(qse_state* st, const qse_op* ops, size_t nops, const double* para
     mark_zero(st);
     execute_program(st, ops, nops, params, nparams, nullptr, nullptr, 0, nullptr);
     if (!st->aux) QSE_CUDA(cudaMalloc(&st->aux, st->size() * 16));
-    double value = run_obs(st, obs, reinterpret_cast<double2*>(st->aux));
+    const ObsRun obs_run = launch_obs(st, obs, reinterpret_cast<double2*>(st->aux));
+    try {   // one synchronisation, at the end of the sweep
+        return adjoint_sweep(st, ops, nops, params, nparams, obs_run, grad);
+    } catch (...) {
+        cudaStreamSynchronize(ctx->stream);   // host_small receives <O> until then
+        throw;
+    }
+}
 
+namespace {
+double adjoint_sweep(qse_state* st, const qse_op* ops, size_t nops, const double* params, size_t nparams,
+                     const ObsRun& obs_run, double* grad)
+{
+    qse_ctx* ctx = st->ctx;
     // reverse sweep over the inverse gates, gradient slots on parameterised ones.
     // Slot sums give 2 Im<l|G|s> for X/Y/Z generators and -2 Im<l|P|s> must be
     // applied for phase types (factor f); occurrences of one parameter with the
@@ -1300,52 +1365,82 @@ double adjoint(qse_state* st, const qse_op* ops, size_t nops, const double* para
     opt.low_lanes = st->n >= kLowLanesQubits;
     const std::shared_ptr<PlanEntry> e = plan_for(st, rev, opt, 2);
     const plan::Plan& pl = e->pl;
-    Uploaded up = upload_plan(ctx, pl, e->use_jit && st->n >= jit::kPreGroupQubits);
+    Uploaded up = upload_plan(ctx, pl, e->use_jit, e->use_jit && st->n >= jit::kPreGroupQubits);
 
-    // occurrence gradients accumulate in scratch2: [nops] | slot partials
-    size_t max_part = 0;
-    for (size_t i = 0; i < pl.passes.size(); ++i)
-        max_part = std::max(max_part, pl.passes[i].slot_src.size() * (size_t(1) << (st->n - pl.passes[i].k)));
-    size_t srcmax = 0;
-    for (auto& p : pl.passes) srcmax = std::max(srcmax, p.slot_src.size());
-    size_t b_occ = align16(nops * 8 + 8), b_part = align16(max_part * 8 + 8), b_src = align16(srcmax * 4 + 4);
-    ctx->scratch2.reserve(b_occ + b_part + b_src * pl.passes.size() + 16);
+    // Bucket gradients accumulate in scratch2: buckets | slot partials | entries |
+    // segments.  Passes are reduced in groups whose partials fit kMaxPartialBytes
+    // (or one by one), the entries of a group sorted by bucket.
+    struct Group {
+        size_t last;                  // its last pass
+        uint32_t seg0, nseg;
+    };
+    std::vector<Group> groups;
+    std::vector<SlotSums> entries;
+    std::vector<uint32_t> seg;
+    std::vector<uint64_t> part_off(pl.passes.size(), 0);
+    uint64_t part = 0, max_part = 0;   // doubles
+    size_t group_begin = 0;
+    auto close_group = [&](size_t last) {
+        std::stable_sort(entries.begin() + std::ptrdiff_t(group_begin), entries.end(),
+                         [](const SlotSums& a, const SlotSums& b) { return a.src < b.src; });
+        Group g{last, uint32_t(seg.size()), 0};
+        for (size_t k = group_begin; k < entries.size(); ++k)
+            if (k == group_begin || entries[k].src != entries[k - 1].src) {
+                seg.push_back(uint32_t(k));
+                ++g.nseg;
+            }
+        seg.push_back(uint32_t(entries.size()));
+        if (g.nseg) groups.push_back(g);
+        group_begin = entries.size();
+        part = 0;
+    };
+    for (size_t i = 0; i < pl.passes.size(); ++i) {
+        const plan::PassProgram& p = pl.passes[i];
+        const uint64_t nb = uint64_t(1) << (st->n - p.k);
+        if (part && (part + p.slot_src.size() * nb) * 8 > kMaxPartialBytes) close_group(i - 1);
+        part_off[i] = part;
+        for (size_t s = 0; s < p.slot_src.size(); ++s)
+            entries.push_back(SlotSums{part + s * nb, uint32_t(nb), uint32_t(p.slot_src[s])});
+        part += p.slot_src.size() * nb;
+        max_part = std::max(max_part, part);
+    }
+    if (!pl.passes.empty()) close_group(pl.passes.size() - 1);
+    const size_t b_occ = align16(buckets.size() * 8 + 8), b_part = align16(max_part * 8 + 8),
+                 b_ent = align16(entries.size() * sizeof(SlotSums)), b_seg = align16(seg.size() * 4);
+    ctx->scratch2.reserve(b_occ + b_part + b_ent + b_seg + 16);
     char* base = static_cast<char*>(ctx->scratch2.ptr);
     double* occ = reinterpret_cast<double*>(base);
-    double* part = reinterpret_cast<double*>(base + b_occ);
-    char* srcbase = base + b_occ + b_part;
-    QSE_CUDA(cudaMemsetAsync(occ, 0, nops * 8 + 8, ctx->stream));
-    // slot -> occurrence maps, one upload
-    {
-        size_t hb = b_src * pl.passes.size() + 16;
-        ctx->host_small2.reserve(hb);
-        char* h = static_cast<char*>(ctx->host_small2.ptr);
-        for (size_t i = 0; i < pl.passes.size(); ++i)
-            std::memcpy(h + i * b_src, pl.passes[i].slot_src.data(), pl.passes[i].slot_src.size() * 4);
-        QSE_CUDA(cudaMemcpyAsync(srcbase, h, b_src * pl.passes.size(), cudaMemcpyHostToDevice, ctx->stream));
-    }
+    double* partial = reinterpret_cast<double*>(base + b_occ);
+    const SlotSums* d_ent = reinterpret_cast<const SlotSums*>(base + b_occ + b_part);
+    const uint32_t* d_seg = reinterpret_cast<const uint32_t*>(base + b_occ + b_part + b_ent);
+    QSE_CUDA(cudaMemsetAsync(occ, 0, buckets.size() * 8 + 8, ctx->stream));
+    // (host_small2 feeds nothing here: its other users synchronise before they return)
+    ctx->host_small2.reserve(b_occ + b_ent + b_seg + 16);
+    double* hocc = static_cast<double*>(ctx->host_small2.ptr);
+    char* h = reinterpret_cast<char*>(hocc) + b_occ;
+    std::memcpy(h, entries.data(), entries.size() * sizeof(SlotSums));
+    std::memcpy(h + b_ent, seg.data(), seg.size() * 4);
+    QSE_CUDA(cudaMemcpyAsync(base + b_occ + b_part, h, b_ent + b_seg, cudaMemcpyHostToDevice, ctx->stream));
     PassRunner runner(st, *e, up, 2, 3);
+    size_t g = 0;
     for (size_t i = 0; i < up.args.size(); ++i) {
-        const tile::PassArgs& a = up.args[i];
-        runner.run(i, reinterpret_cast<double2*>(st->aux), part);
-        if (a.nslots) {
-            uint64_t nb = uint64_t(1) << (st->n - a.k);
-            unsigned g = std::min<unsigned>(a.nslots, unsigned(ctx->num_sms) * 4);
-            k_reduce_slots<<<g, kRB, 0, ctx->stream>>>(part, a.nslots, nb,
-                                                        reinterpret_cast<const int32_t*>(srcbase + i * b_src), occ);
+        runner.run(i, reinterpret_cast<double2*>(st->aux), partial + part_off[i]);
+        if (g < groups.size() && groups[g].last == i) {
+            k_reduce_slots<<<groups[g].nseg, kRB, 0, ctx->stream>>>(partial, d_ent, d_seg + groups[g].seg0, occ);
             QSE_CUDA(cudaGetLastError());
             count_launch(ctx);
+            ++g;
         }
     }
     for (uint32_t q = 0; q < st->n; ++q) st->perm[q] = pl.perm_final[q];
     st->touch();
-    std::vector<double> hocc(nops);
-    QSE_CUDA(cudaMemcpyAsync(hocc.data(), occ, nops * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    QSE_CUDA(cudaMemcpyAsync(hocc, occ, buckets.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
     QSE_CUDA(cudaStreamSynchronize(ctx->stream));
     for (size_t p = 0; p < nparams; ++p) grad[p] = 0.0;
     for (size_t b = 0; b < buckets.size(); ++b)
         if (size_t(buckets[b].first) < nparams) grad[buckets[b].first] += buckets[b].second * hocc[b];
-    return value;
+    return obs_run.value();
 }
+}  // namespace
 
 }  // namespace qse

@@ -67,13 +67,15 @@ struct qse_ctx {
     unsigned* status_dev = nullptr;
     // scratch shared by the calls on this context (single host thread, like the reference backend)
     qse::DevBuf plan_buf;    // uploaded pass programs
-    qse::HostBuf plan_host;  // pinned staging for the pass programs
+    qse::HostBuf plan_host[2];  // pinned staging for the pass programs, used in turn
+    int plan_turn = 0;
     qse::DevBuf scratch;     // reductions, sampling, noise decisions
     qse::DevBuf scratch2;
     qse::DevBuf gv_buf;      // per-tile group values of the pass being launched (precomputed)
     qse::HostBuf host_small; // pinned small results
     qse::HostBuf host_small2;
-    cudaEvent_t plan_event = nullptr;  // last H2D copy out of plan_host
+    cudaEvent_t plan_event[2] = {};    // last H2D copy out of plan_host[i]
+    cudaEvent_t small_event = nullptr; // last H2D copy out of host_small that nothing waited for
     cudaEvent_t slots[64] = {};        // qse_ctx_record / qse_ctx_elapsed
     // qse_ctx_time_passes: event pairs around every fused-pass launch
     bool time_passes = false;
