@@ -123,11 +123,13 @@ constexpr uint32_t kMaxThreads = 512;
 // gives up: about a second, far beyond any pass of a circuit that fits
 constexpr uint32_t kDefaultWaitPolls = 1u << 21;
 
-// exchange buffer | group values | per-warp gradient partials | warp sums
-size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads)
+// exchange buffer | group values | angle accumulators | per-warp gradient
+// partials | warp sums
+size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb)
 {
     const size_t nwarps = threads / 32;
-    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + size_t(max_slots) * nwarps * 8 + nwarps * 8;
+    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + size_t(rb) * threads * 8 +
+           size_t(max_slots) * nwarps * 8 + nwarps * 8;
 }
 
 // ------------------------------------------------------------------ device
@@ -178,7 +180,7 @@ __device__ __forceinline__ double block_sum(double v, double* red, uint32_t nwar
 
 template <int RB>
 __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint32_t tile, double2* xbuf, double2* gval,
-                                         double* wpart, double* red, uint8_t* s_tile, uint32_t nwarps)
+                                         double* acc, double* wpart, double* red, uint32_t nwarps)
 {
     constexpr int R = 1 << RB;
     const uint32_t tid = threadIdx.x;
@@ -189,15 +191,18 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     const bool rev = flags & F_REV;
 
     __syncthreads();  // the previous tile's users of the shared tables are done
-    if (tid < 16) s_tile[tid] = P.tile_phys[tid];
     group_values(A.groups + P.grp0, P.ngroups, A.terms + P.term0, obase, gval);
     if (rev)
         for (uint32_t i = tid; i < nslots * nwarps; i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const bool active = tid < (1u << (k - RB));
-    LayoutState<RB> L;
-    load_layout<RB>(L, A.layouts + P.lay0 + P.layout0, s_tile, k, obase, tid);
+    // circuits have at most 30 qubits: 32-bit amplitude indices
+    const plan::LayoutRec* lay = A.layouts + P.lay0 + P.layout0;
+    uint32_t rg[RB];
+#pragma unroll
+    for (int i = 0; i < RB; ++i) rg[i] = 1u << lay->preg[i];
+    uint32_t base = thread_base<uint32_t>(lay, uint32_t(obase), tid);
     double2* psi = A.pool + C.psi;
     double2* lam = A.pool + C.lam;
 
@@ -208,7 +213,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         a[0][j] = make_double2(0.0, 0.0);
         a[1][j] = make_double2(0.0, 0.0);
         if (!active) continue;
-        const uint64_t idx = gidx<RB>(L, j);
+        const uint32_t idx = reg_index<RB>(base, rg, j);
         if (flags & F_ZERO) a[0][j] = make_double2(idx == 0 ? 1.0 : 0.0, 0.0);
         else a[0][j] = __ldcg(psi + idx);
         if (flags & F_LAMBDA) {
@@ -220,14 +225,17 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         }
     }
 
-    const OpsEnv E{A.ops + P.op0, P.nops, A.layouts + P.lay0, A.mats + 8 * size_t(P.mat0), s_tile, k, obase,
-                   xbuf, gval, wpart, nwarps};
-    run_ops<RB, 2>(E, L, a, rev ? 2 : 1, active);
+    const OpsEnv E{A.ops + P.op0, P.nops, A.layouts + P.lay0, A.mats + 8 * size_t(P.mat0), obase,
+                   xbuf, gval, wpart, nwarps, acc};
+    lay = run_ops<RB, 2>(E, lay, a, rev ? 2 : 1, active);
 
     if (!(flags & F_NOSTORE) && active) {
 #pragma unroll
+        for (int i = 0; i < RB; ++i) rg[i] = 1u << lay->preg[i];
+        base = thread_base<uint32_t>(lay, uint32_t(obase), tid);
+#pragma unroll
         for (int j = 0; j < R; ++j) {
-            const uint64_t idx = gidx<RB>(L, j);
+            const uint32_t idx = reg_index<RB>(base, rg, j);
             __stcg(psi + idx, a[0][j]);
             if (rev) __stcg(lam + idx, a[1][j]);
         }
@@ -247,20 +255,23 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     }
 }
 
-// Register budget: WIDE = 0 caps the kernel at 128 registers per thread (two
-// CTAs of 256 threads per SM, a few spills); WIDE = 1 lets it use up to 255
-// (CTAs of at most 256 threads, one per SM).  The autotuner picks by measurement.
+// Register budget: WIDE = 0 caps the kernel at 128 registers per thread for 4 or
+// 8 amplitudes per thread and state (two CTAs of 256 threads per SM) and 168 for
+// 16 (three CTAs of 128); WIDE = 1 lets it use up to 255 (CTAs of at most 256
+// threads).  The autotuner picks by measurement.
 template <int RB, int WIDE>
-__global__ void __launch_bounds__(WIDE ? 256 : kMaxThreads, 1) k_batch(const __grid_constant__ BatchArgs A)
+__global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB == 4 && !WIDE ? 3 : 1)
+    k_batch(const __grid_constant__ BatchArgs A)
 {
     extern __shared__ double2 smem[];
     const uint32_t tid = threadIdx.x;
     const uint32_t nwarps = blockDim.x >> 5;
     double2* xbuf = smem;
     double2* gval = smem + (size_t(1) << A.kmax);
-    double* wpart = reinterpret_cast<double*>(gval + A.max_groups);
+    double* acc = reinterpret_cast<double*>(gval + A.max_groups);
+    double* wpart = acc + RB * blockDim.x;
     double* red = wpart + size_t(A.max_slots) * nwarps;
-    __shared__ uint8_t s_tile[16];
+    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = 0.0;
     __shared__ uint32_t s_cur, s_next;
     __shared__ int s_ok;
 
@@ -281,7 +292,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : kMaxThreads, 1) k_batch(const __g
         if (!s_ok) break;
         for (uint32_t p = 0; p < item.npass; ++p)
             for (uint32_t t = 0; t < item.ntile; ++t)
-                run_tile<RB>(A, item.pass + p, item.tile + t, xbuf, gval, wpart, red, s_tile, nwarps);
+                run_tile<RB>(A, item.pass + p, item.tile + t, xbuf, gval, acc, wpart, red, nwarps);
         // publish: every thread's stores are visible GPU-wide before the counter moves
         __threadfence();
         __syncthreads();
@@ -356,10 +367,25 @@ struct Config {
     uint32_t wide = 0;         // 1: up to 255 registers per thread (threads <= 256); 0: 128
 };
 
-const void* kernel_of(const Config& c)
+// How a configuration's tiles (2^(log2(threads) + reg_bits) amplitudes) run:
+// with reg_bits 3, from 64 threads on, 16 amplitudes per thread and state in CTAs
+// of half the threads.  The interpreter's own instructions (nine in ten with 8
+// per thread) are per warp and op, so a tile then takes half of them, and a
+// layout exchange serves four qubits instead of three.
+struct Shape {
+    uint32_t threads, rb;
+    const void* kernel;
+};
+
+Shape shape_of(const Config& c)
 {
-    if (c.rb == 3) return c.wide ? reinterpret_cast<const void*>(k_batch<3, 1>) : reinterpret_cast<const void*>(k_batch<3, 0>);
-    return c.wide ? reinterpret_cast<const void*>(k_batch<2, 1>) : reinterpret_cast<const void*>(k_batch<2, 0>);
+    auto fn = [](void (*k)(BatchArgs)) { return reinterpret_cast<const void*>(k); };
+    if (c.rb == 3 && c.threads >= 64) {
+        const uint32_t t = c.threads / 2;
+        return Shape{t, 4, c.wide || t > 128 ? fn(k_batch<4, 1>) : fn(k_batch<4, 0>)};
+    }
+    if (c.rb == 3) return Shape{c.threads, 3, fn(k_batch<3, 0>)};
+    return Shape{c.threads, 2, c.wide ? fn(k_batch<2, 1>) : fn(k_batch<2, 0>)};
 }
 
 struct CircuitHost {
@@ -491,6 +517,7 @@ void build(qse_batch* b)
     qse_ctx* ctx = b->ctx;
     const Config& cf = b->cfg;
     const uint32_t kcfg = log2u(cf.threads) + cf.rb;
+    const Shape shape = shape_of(cf);
     drop_graph(b);
     b->built = false;
 
@@ -515,7 +542,7 @@ void build(qse_batch* b)
         const CircuitHost& ch = b->circs[ci];
         const uint32_t w = ch.w;
         plan::Options opt;
-        opt.rb = cf.rb;
+        opt.rb = shape.rb;
         opt.k = std::min(kcfg, w);
         opt.max_gates = cf.max_gates;
         opt.max_terms = 512;
@@ -571,7 +598,6 @@ void build(qse_batch* b)
         vpart_total += c.nvpart;
 
         const size_t nf = pf.passes.size(), nall = nf + pr.passes.size();
-        const bool multi = nt > cf.chain_tiles;
         for (size_t j = 0; j < nall; ++j) {
             const bool isrev = j >= nf;
             const plan::PassProgram& P = isrev ? pr.passes[j - nf] : pf.passes[j];
@@ -588,7 +614,7 @@ void build(qse_batch* b)
             bp.k = P.k;
             bp.ntiles = nt;
             bp.circ = uint32_t(ci);
-            bp.wait = (j > 0 && multi) ? int32_t(passes.size() - 1) : -1;
+            bp.wait = j > 0 ? int32_t(passes.size() - 1) : -1;   // (a single item's passes wait for nothing: below)
             std::memcpy(bp.tile_phys, P.tile_phys, 16);
             if (j == 0) bp.flags |= F_ZERO;
             if (isrev) {
@@ -630,7 +656,6 @@ void build(qse_batch* b)
             mats.insert(mats.end(), P.mats.begin(), P.mats.end());
             passes.push_back(bp);
             visits += nt;
-            if (multi) hbm += amps * (isrev ? 64u : 32u);
         }
         // a reverse-only circuit (no forward pass) starts its reverse sweep from |0..0>
         if (nf == 0 && nall > 0) passes[first_pass[ci]].flags |= F_ZERO;
@@ -658,13 +683,47 @@ void build(qse_batch* b)
         }
     }
 
+    // shared memory and grid
+    const size_t smem = smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb);
+    if (smem + 64 > ctx->smem_optin)
+        fail(QSE_ERR_SIZE, "batch: a pass needs " + std::to_string(smem) +
+                               " B of shared memory; lower max_gates or the tile size");
+    const void* kfn = shape.kernel;
+    {
+        cudaFuncAttributes fa{};
+        QSE_CUDA(cudaFuncGetAttributes(&fa, kfn));
+        QSE_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(ctx->smem_optin - fa.sharedSizeBytes)));
+    }
+    int occ_blocks = 0;
+    QSE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blocks, kfn, int(shape.threads), smem));
+    if (occ_blocks < 1) fail(QSE_ERR_SIZE, "batch: kernel configuration does not fit on an SM");
+    uint32_t per_sm = uint32_t(occ_blocks);
+    if (cf.ctas_per_sm) per_sm = std::min(per_sm, cf.ctas_per_sm);
+    const uint64_t resident = uint64_t(ctx->num_sms) * per_sm;
+    b->smem = smem;
+
+    // Circuits of at most chain_tiles tiles are single items, unless one alone
+    // would keep its CTA busy for more than twice the batch's share of a CTA: the
+    // others would then wait for it (48 circuits of 6 to 13 qubits: 1.95 -> 0.81 ms).
+    std::vector<char> single(b->circs.size(), 0);
+    for (size_t ci = 0; ci < b->circs.size(); ++ci) {
+        const uint64_t own = uint64_t(npass[ci]) * ntiles[ci];
+        single[ci] = ntiles[ci] == 1 || (ntiles[ci] <= cf.chain_tiles && own * resident <= 2 * visits);
+        for (uint32_t j = 0; j < npass[ci]; ++j) {
+            BPass& p = passes[first_pass[ci] + j];
+            if (single[ci]) p.wait = -1;
+            else hbm += (uint64_t(1) << b->circs[ci].w) * ((p.flags & F_REV) ? 64u : 32u);
+        }
+    }
+
     // work queue: single-CTA circuits first (longest first), then level-major tiles
     std::vector<BItem> items;
     {
         std::vector<size_t> chains, multis;
         for (size_t ci = 0; ci < b->circs.size(); ++ci) {
             if (npass[ci] == 0) continue;
-            (ntiles[ci] <= cf.chain_tiles ? chains : multis).push_back(ci);
+            (single[ci] ? chains : multis).push_back(ci);
         }
         std::stable_sort(chains.begin(), chains.end(), [&](size_t x, size_t y) {
             return uint64_t(npass[x]) * ntiles[x] * (uint64_t(1) << b->circs[x].w) >
@@ -681,25 +740,7 @@ void build(qse_batch* b)
         if (items.size() > 0xffffff00ull) fail(QSE_ERR_SIZE, "batch: work queue too long");
     }
 
-    // shared memory and grid
-    const size_t smem = smem_bytes(kmax, max_groups, max_slots, cf.threads);
-    if (smem + 64 > ctx->smem_optin)
-        fail(QSE_ERR_SIZE, "batch: a pass needs " + std::to_string(smem) +
-                               " B of shared memory; lower max_gates or the tile size");
-    const void* kfn = kernel_of(cf);
-    {
-        cudaFuncAttributes fa{};
-        QSE_CUDA(cudaFuncGetAttributes(&fa, kfn));
-        QSE_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(ctx->smem_optin - fa.sharedSizeBytes)));
-    }
-    int occ_blocks = 0;
-    QSE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blocks, kfn, int(cf.threads), smem));
-    if (occ_blocks < 1) fail(QSE_ERR_SIZE, "batch: kernel configuration does not fit on an SM");
-    uint32_t per_sm = uint32_t(occ_blocks);
-    if (cf.ctas_per_sm) per_sm = std::min(per_sm, cf.ctas_per_sm);
-    b->grid = unsigned(std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, std::max<size_t>(items.size(), 1)));
-    b->smem = smem;
+    b->grid = unsigned(std::min<uint64_t>(resident, std::max<size_t>(items.size(), 1)));
 
     // one blob for everything read-only (plus the patched ops / terms)
     std::vector<char> blob;
@@ -806,12 +847,9 @@ void enqueue(qse_batch* b)
         QSE_CUDA(cudaGetLastError());
     }
     if (b->args.nitems) {
-        const Config& c = b->cfg;
-        if (c.rb == 3 && c.wide) k_batch<3, 1><<<b->grid, c.threads, b->smem, s>>>(b->args);
-        else if (c.rb == 3) k_batch<3, 0><<<b->grid, c.threads, b->smem, s>>>(b->args);
-        else if (c.wide) k_batch<2, 1><<<b->grid, c.threads, b->smem, s>>>(b->args);
-        else k_batch<2, 0><<<b->grid, c.threads, b->smem, s>>>(b->args);
-        QSE_CUDA(cudaGetLastError());
+        const Shape sh = shape_of(b->cfg);
+        void* args[] = {&b->args};
+        QSE_CUDA(cudaLaunchKernel(sh.kernel, dim3(b->grid), dim3(sh.threads), args, b->smem, s));
     }
     if (b->nfins) {
         k_fin_slots<<<b->nfins, 128, 0, s>>>(b->fins, b->args.part, b->slot_occ, b->occ);

@@ -365,9 +365,15 @@ private:
     uint32_t add_layout(const int* prev)
     {
         LayoutRec rec{};
-        for (uint32_t i = 0; i < P.rb; ++i) rec.reg[i] = uint8_t(reg_[i]);
+        for (uint32_t i = 0; i < P.rb; ++i) {
+            rec.reg[i] = uint8_t(reg_[i]);
+            rec.preg[i] = P.tile_phys[reg_[i]];
+        }
         rec.nthr = uint8_t(nthr_);
-        for (int t = 0; t < nthr_; ++t) rec.thr[t] = uint8_t(thr_[t]);
+        for (int t = 0; t < nthr_; ++t) {
+            rec.thr[t] = uint8_t(thr_[t]);
+            rec.pthr[t] = P.tile_phys[thr_[t]];
+        }
         uint32_t s[16] = {0};
         if (prev && nthr_ >= 3) {
             int pl[3], nl[3], np = 0;
@@ -399,6 +405,16 @@ private:
             }
         }
         for (uint32_t b = 0; b < 16; ++b) rec.L[b] = uint16_t((1u << b) ^ (b >= 3 ? s[b] : 0u));
+        for (uint32_t i = 0; i < P.rb; ++i) rec.rreg[i] = rec.L[reg_[i]];
+        for (int t = 0; t < nthr_; ++t) rec.rthr[t] = rec.L[thr_[t]];
+        if (prev) {
+            uint32_t t = 0;
+            for (uint32_t b = 0; b < P.k; ++b) {
+                const int* r = std::find(prev, prev + P.rb, int(b));
+                if (r != prev + P.rb) rec.wreg[r - prev] = rec.L[b];
+                else rec.wthr[t++] = rec.L[b];
+            }
+        }
         P.layouts.push_back(rec);
         return uint32_t(P.layouts.size() - 1);
     }

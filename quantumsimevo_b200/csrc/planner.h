@@ -56,14 +56,24 @@ struct KOp {
 };
 static_assert(sizeof(KOp) == 32, "KOp layout");
 
-struct LayoutRec {
-    uint8_t reg[5];    // tile-local bits held in registers (register index bit i <-> reg[i]; rb <= 5)
-    uint8_t nthr;      // number of thread-index bits
-    uint8_t pad[2];
-    uint16_t L[16];    // shared-memory slot image of every tile-local bit (XOR-linear map)
-    uint8_t thr[16];   // tile-local bit of thread-index bit t (ascending), t < nthr
+// Per-thread-bit entries beyond the layout's thread bits are 0: the interpreter
+// always walks kThrBits of them.  wthr/wreg and rthr/rreg are the slot images of
+// what a thread writes (the layout before) and reads (this one) in the exchange
+// into this layout, so that it does not look them up through two tables.
+constexpr uint32_t kThrBits = 10;   // 12 tile qubits, 2 of them in registers
+struct alignas(16) LayoutRec {
+    uint16_t L[16];        // shared-memory slot image of every tile-local bit (XOR-linear map)
+    uint16_t wthr[16];
+    uint16_t rthr[16];
+    uint16_t wreg[8], rreg[8];
+    uint8_t reg[8];        // tile-local bits held in registers (register index bit i <-> reg[i]; rb <= 5)
+    uint8_t preg[8];       // their physical qubits
+    uint8_t thr[16];       // tile-local bit of thread-index bit t (ascending), t < nthr
+    uint8_t pthr[16];      // their physical qubits
+    uint8_t nthr;          // number of thread-index bits
+    uint8_t pad[15];
 };
-static_assert(sizeof(LayoutRec) == 56, "LayoutRec layout");
+static_assert(sizeof(LayoutRec) == 192, "LayoutRec layout");
 
 struct TermRec {       // one diagonal term: angle theta if all outer bits of ocond are set
     uint64_t ocond;

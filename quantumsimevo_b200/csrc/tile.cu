@@ -36,11 +36,10 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
     const uint32_t tsize = 1u << A.k;
     double2* xbuf = smem;
     double2* gval = smem + tsize;
-    double* wpart = reinterpret_cast<double*>(gval + A.ngroups);
+    double* acc = reinterpret_cast<double*>(gval + A.ngroups);
+    double* wpart = acc + RB * blockDim.x;
     const uint32_t nwarps = (blockDim.x + 31) >> 5;
-
-    __shared__ uint8_t s_tile[16];
-    for (uint32_t i = tid; i < 16; i += blockDim.x) s_tile[i] = A.tile_phys[i];
+    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = 0.0;
 
     const uint64_t obase = tile_base(blockIdx.x, A.outer_mask);
     group_values(A.groups, A.ngroups, A.terms, obase, gval);
@@ -48,23 +47,26 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
         for (uint32_t i = tid; i < A.nslots * nwarps; i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
-    LayoutState<RB> L;
-    load_layout<RB>(L, A.layouts + A.layout0, s_tile, A.k, obase, tid);
-
+    const plan::LayoutRec* lay = A.layouts + A.layout0;
+    uint64_t rg[RB];
+    for (int i = 0; i < RB; ++i) rg[i] = uint64_t(1) << lay->preg[i];
+    uint64_t base = thread_base<uint64_t>(lay, obase, tid);
     double2 a[NS][R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-        uint64_t idx = gidx<RB>(L, j);
+        uint64_t idx = reg_index<RB>(base, rg, j);
         a[0][j] = A.psi[idx];
         if (NS == 2) a[NS - 1][j] = A.lam[idx];
     }
 
-    OpsEnv E{A.ops, A.nops, A.layouts, A.mats, s_tile, A.k, obase, xbuf, gval, wpart, nwarps};
-    run_ops<RB, NS>(E, L, a, NS, true);
+    OpsEnv E{A.ops, A.nops, A.layouts, A.mats, obase, xbuf, gval, wpart, nwarps, acc};
+    lay = run_ops<RB, NS>(E, lay, a, NS, true);
 
+    for (int i = 0; i < RB; ++i) rg[i] = uint64_t(1) << lay->preg[i];
+    base = thread_base<uint64_t>(lay, obase, tid);
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-        uint64_t idx = gidx<RB>(L, j);
+        uint64_t idx = reg_index<RB>(base, rg, j);
         A.psi[idx] = a[0][j];
         if (NS == 2) A.lam[idx] = a[NS - 1][j];
     }
@@ -125,7 +127,7 @@ void pass_timer_end(qse_ctx* ctx, cudaEvent_t stop)
 size_t pass_smem_bytes(uint32_t k, uint32_t ngroups, uint32_t nslots, uint32_t rb, int nstates)
 {
     size_t threads = size_t(1) << (k - rb);
-    size_t b = (size_t(1) << k) * 16 + size_t(ngroups) * 16;
+    size_t b = (size_t(1) << k) * 16 + size_t(ngroups) * 16 + size_t(rb) * threads * 8;
     if (nstates == 2) b += size_t(nslots) * ((threads + 31) / 32) * 8;
     return b;
 }

@@ -189,54 +189,37 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-template <int RB>
-struct LayoutState {
-    int reg[RB];                     // tile-local bits in registers
-    uint64_t rg[RB];                 // their physical masks
-    uint64_t gbase;                  // physical index of register 0 of this thread
-    const plan::LayoutRec* rec;      // thread-bit list of the layout
-};
-
-template <int RB>
-__device__ __forceinline__ void load_layout(LayoutState<RB>& L, const plan::LayoutRec* rec, const uint8_t* tphys,
-                                            uint32_t /*k*/, uint64_t obase, uint32_t tid)
+// XOR of the 16-bit images img[t] over the set bits t < kThrBits of tid, two
+// per word (img 16-byte aligned).
+__device__ __forceinline__ uint32_t slot_of(const uint16_t* img, uint32_t tid)
 {
-    L.rec = rec;
+    const uint4 w = *reinterpret_cast<const uint4*>(img);
+    const uint32_t v[5] = {w.x, w.y, w.z, w.w, *reinterpret_cast<const uint32_t*>(img + 8)};
+    static_assert(plan::kThrBits == 10, "five words of two images");
+    uint32_t s = 0;
 #pragma unroll
-    for (int i = 0; i < RB; ++i) {
-        L.reg[i] = rec->reg[i];
-        L.rg[i] = uint64_t(1) << tphys[L.reg[i]];
-    }
-    uint64_t g = obase;
-    const uint32_t nthr = rec->nthr;
-    for (uint32_t t = 0; t < nthr; ++t)
-        if ((tid >> t) & 1u) g |= uint64_t(1) << tphys[rec->thr[t]];
-    L.gbase = g;
+    for (int p = 0; p < 5; ++p)
+        s ^= v[p] & (((tid >> (2 * p)) & 1u) * 0xffffu | ((tid >> (2 * p + 1)) & 1u) * 0xffff0000u);
+    return (s ^ (s >> 16)) & 0xffffu;
 }
 
-// shared-memory slot of register 0 and per-register-bit slot images under map Lm
-template <int RB>
-__device__ __forceinline__ uint32_t slot_base(const LayoutState<RB>& L, const uint16_t* Lm, uint32_t /*k*/,
-                                              uint32_t tid, uint32_t (&sreg)[RB])
+// index of register 0 of thread tid in layout r: the outer bits and its thread bits
+template <class I>
+__device__ __forceinline__ I thread_base(const plan::LayoutRec* r, I obase, uint32_t tid)
 {
-    uint32_t sb = 0;
-    const plan::LayoutRec* r = L.rec;
-    const uint32_t nthr = r->nthr;
-    for (uint32_t t = 0; t < nthr; ++t)
-        if ((tid >> t) & 1u) sb ^= Lm[r->thr[t]];
+    I g = obase;
 #pragma unroll
-    for (int i = 0; i < RB; ++i) sreg[i] = Lm[L.reg[i]];
-    return sb;
+    for (uint32_t t = 0; t < plan::kThrBits; ++t) g |= I((tid >> t) & 1u) << r->pthr[t];
+    return g;
 }
 
-template <int RB>
-__device__ __forceinline__ uint64_t gidx(const LayoutState<RB>& L, int j)
+template <int RB, class I>
+__device__ __forceinline__ I reg_index(I base, const I (&rg)[RB], int j)
 {
-    uint64_t idx = L.gbase;
 #pragma unroll
     for (int i = 0; i < RB; ++i)
-        if ((j >> i) & 1) idx |= L.rg[i];
-    return idx;
+        if ((j >> i) & 1) base |= rg[i];
+    return base;
 }
 
 template <int RB>
@@ -249,14 +232,13 @@ __device__ __forceinline__ uint32_t sidx(uint32_t sb, const uint32_t (&sreg)[RB]
     return s;
 }
 
+// acc: the thread's accumulated angle of register bit p (shared memory)
 template <int RB, int NS>
-__device__ __forceinline__ void flush_reg(int p, double (&acc)[RB], double2 (&a)[NS][1 << RB], int nact)
+__device__ __forceinline__ void flush_reg(int p, double* acc, double2 (&a)[NS][1 << RB], int nact)
 {
-    double v = 0.0;
-#pragma unroll
-    for (int i = 0; i < RB; ++i)
-        if (i == p) { v = acc[i]; acc[i] = 0.0; }
+    const double v = *acc;
     if (v != 0.0) {
+        *acc = 0.0;
         double s, c;
         sincos(v, &s, &c);
         OpPhase1 ph{make_double2(c, s)};
@@ -308,31 +290,29 @@ struct OpsEnv {
     uint32_t nops;
     const plan::LayoutRec* layouts;   // layout indices of the program are relative to this
     const double* mats;               // K_U matrix indices are relative to this
-    const uint8_t* tile_phys;         // shared-memory copy of the pass's tile qubits
-    uint32_t k;
     uint64_t obase;
     double2* xbuf;                    // 2^k slots
     const double2* gval;              // group values of this CTA
     double* wpart;                    // [slot][warp] gradient partials (NS == 2)
     uint32_t nwarps;
+    double* acc;                      // angle accumulators, [register bit][thread] (zero on entry and exit)
 };
 
-// Executes a pass program on the registers a[NS][R].  nact states take part
+// Executes a pass program on the registers a[NS][R], which hold layout `lay` and
+// leave in the layout returned.  nact states take part
 // (1: only |psi>, forward; NS: the adjoint sweep on |psi> and |lambda>).
 // Threads with active == false hold zeros, never touch the exchange buffer
 // and add nothing to the gradient partials; they only join the barriers
 // (a CTA wider than the tile of a small state).
 template <int RB, int NS>
-__device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, double2 (&a)[NS][1 << RB], int nact,
-                                        bool active)
+__device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const plan::LayoutRec* lay,
+                                                         double2 (&a)[NS][1 << RB], int nact, bool active)
 {
     constexpr int R = 1 << RB;
     const uint32_t tid = threadIdx.x;
     const uint32_t warp = tid >> 5, lane = tid & 31;
     double acc_thr = 0.0;
-    double acc[RB];
-#pragma unroll
-    for (int i = 0; i < RB; ++i) acc[i] = 0.0;
+    double* const acc = E.acc + tid;
 
     KOp nxt = E.nops ? E.ops[0] : KOp{};
     for (uint32_t i = 0; i < E.nops; ++i) {
@@ -394,12 +374,7 @@ __device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, dou
             if (tc) acc_thr += E.gval[op.g].x;
             break;
         case plan::K_ACC_REG: {
-            if (tc) {
-                double v = E.gval[op.g].x;
-#pragma unroll
-                for (int r = 0; r < RB; ++r)
-                    if (r == op.p) acc[r] += v;
-            }
+            if (tc) acc[op.p * blockDim.x] += E.gval[op.g].x;
             break;
         }
         case plan::K_PHD: {
@@ -412,12 +387,12 @@ __device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, dou
             break;
         }
         case plan::K_FLUSH_REG:
-            flush_reg<RB, NS>(op.p, acc, a, nact);
+            flush_reg<RB, NS>(op.p, acc + op.p * blockDim.x, a, nact);
             break;
         case plan::K_FLUSH_ALL: {
 #pragma unroll
             for (int r = 0; r < RB; ++r)
-                if ((op.f >> r) & 1) flush_reg<RB, NS>(r, acc, a, nact);
+                if ((op.f >> r) & 1) flush_reg<RB, NS>(r, acc + r * blockDim.x, a, nact);
             double2 e = make_double2(op.a, op.b);
             if (acc_thr != 0.0) {
                 double s, c;
@@ -435,13 +410,14 @@ __device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, dou
             break;
         }
         case plan::K_TRANSPOSE: {
-            const plan::LayoutRec* nrec = E.layouts + op.g;
-            const uint16_t* Lm = nrec->L;
+            lay = E.layouts + op.g;
+            const uint32_t sbw = slot_of(lay->wthr, tid), sbr = slot_of(lay->rthr, tid);
             uint32_t sreg_w[RB], sreg_r[RB];
-            uint32_t sbw = slot_base<RB>(L, Lm, E.k, tid, sreg_w);
-            LayoutState<RB> N;
-            load_layout<RB>(N, nrec, E.tile_phys, E.k, E.obase, tid);
-            uint32_t sbr = slot_base<RB>(N, Lm, E.k, tid, sreg_r);
+#pragma unroll
+            for (int i = 0; i < RB; ++i) {
+                sreg_w[i] = lay->wreg[i];
+                sreg_r[i] = lay->rreg[i];
+            }
 #pragma unroll
             for (int st = 0; st < NS; ++st) {
                 if (st < nact) {
@@ -455,7 +431,6 @@ __device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, dou
                         for (int j = 0; j < R; ++j) a[st][j] = E.xbuf[sidx<RB>(sbr, sreg_r, j)];
                 }
             }
-            L = N;
             break;
         }
         case plan::K_GRAD_X:
@@ -494,6 +469,7 @@ __device__ __forceinline__ void run_ops(const OpsEnv& E, LayoutState<RB>& L, dou
             break;
         }
     }
+    return lay;
 }
 
 }  // namespace dev
