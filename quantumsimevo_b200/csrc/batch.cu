@@ -72,13 +72,19 @@ struct BCirc {
     double value0;               // <O> when the circuit has no gates (|0..0>)
 };
 
+struct BTerm {                   // a diagonal term as its unit phase (cos, sin) of the bound angle
+    double2 e;
+    uint64_t ocond;
+    uint64_t pad;
+};
+
 struct BItem {
     uint32_t pass, npass;        // consecutive passes [pass, pass + npass)
     uint32_t tile, ntile;        // tiles [tile, tile + ntile) of each
 };
 
 struct BPatch {                  // angle = theta0 + coeff * params[param]
-    uint32_t dst, kind;          // kind 0: ops[dst].(a, b) = (cos, sin)(angle / 2); 1: terms[dst].theta = angle
+    uint32_t dst, kind;          // kind 0: ops[dst].(a, b) = (cos, sin)(angle / 2); 1: terms[dst].e = (cos, sin)(angle)
     int32_t param, pad;
     double theta0, coeff;
 };
@@ -99,7 +105,7 @@ struct BatchArgs {
     const BPass* passes;
     const plan::KOp* ops;
     const plan::LayoutRec* layouts;
-    const plan::TermRec* terms;
+    const BTerm* terms;
     const plan::GroupRec* groups;
     const double* mats;
     const BCirc* circs;
@@ -123,13 +129,13 @@ constexpr uint32_t kMaxThreads = 512;
 // gives up: about a second, far beyond any pass of a circuit that fits
 constexpr uint32_t kDefaultWaitPolls = 1u << 21;
 
-// exchange buffer | group values | angle accumulators | per-warp gradient
-// partials | warp sums
+// exchange buffer | group values | phase accumulators | gradient partials | warp
+// sums
 size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb)
 {
     const size_t nwarps = threads / 32;
-    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + size_t(rb) * threads * 8 +
-           size_t(max_slots) * nwarps * 8 + nwarps * 8;
+    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + size_t(rb) * threads * 16 +
+           size_t(max_slots) * tile::dev::wpart_stride(uint32_t(nwarps)) * 8 + nwarps * 8;
 }
 
 // ------------------------------------------------------------------ device
@@ -180,7 +186,7 @@ __device__ __forceinline__ double block_sum(double v, double* red, uint32_t nwar
 
 template <int RB>
 __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint32_t tile, double2* xbuf, double2* gval,
-                                         double* acc, double* wpart, double* red, uint32_t nwarps)
+                                         double2* acc, double* wpart, double* red, uint32_t nwarps)
 {
     constexpr int R = 1 << RB;
     const uint32_t tid = threadIdx.x;
@@ -191,9 +197,18 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     const bool rev = flags & F_REV;
 
     __syncthreads();  // the previous tile's users of the shared tables are done
-    group_values(A.groups + P.grp0, P.ngroups, A.terms + P.term0, obase, gval);
+    // per-CTA value of every diagonal group: the product of the phases of its
+    // terms whose outer condition holds (bound once per run: no sincos per tile)
+    for (uint32_t g = tid; g < P.ngroups; g += blockDim.x) {
+        const plan::GroupRec gr = A.groups[P.grp0 + g];
+        const BTerm* t = A.terms + P.term0 + gr.first;
+        double2 v = make_double2(1.0, 0.0);
+        for (uint32_t i = 0; i < gr.count; ++i)
+            if ((obase & t[i].ocond) == t[i].ocond) v = cmul(v, t[i].e);
+        gval[g] = v;
+    }
     if (rev)
-        for (uint32_t i = tid; i < nslots * nwarps; i += blockDim.x) wpart[i] = 0.0;
+        for (uint32_t i = tid; i < nslots * wpart_stride(nwarps); i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const bool active = tid < (1u << (k - RB));
@@ -247,11 +262,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     if (rev && nslots) {
         __syncthreads();
         double* out = A.part + P.part0 + uint64_t(tile) * nslots;
-        for (uint32_t s = tid; s < nslots; s += blockDim.x) {
-            double v = 0.0;
-            for (uint32_t w = 0; w < nwarps; ++w) v += wpart[s * nwarps + w];
-            out[s] = v;
-        }
+        for (uint32_t s = tid; s < nslots; s += blockDim.x) out[s] = slot_sum(wpart + s * wpart_stride(nwarps), nwarps);
     }
 }
 
@@ -268,10 +279,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB =
     const uint32_t nwarps = blockDim.x >> 5;
     double2* xbuf = smem;
     double2* gval = smem + (size_t(1) << A.kmax);
-    double* acc = reinterpret_cast<double*>(gval + A.max_groups);
-    double* wpart = acc + RB * blockDim.x;
-    double* red = wpart + size_t(A.max_slots) * nwarps;
-    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = 0.0;
+    double2* acc = gval + A.max_groups;
+    double* wpart = reinterpret_cast<double*>(acc + RB * blockDim.x);
+    double* red = wpart + size_t(A.max_slots) * wpart_stride(nwarps);
+    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = make_double2(1.0, 0.0);
     __shared__ uint32_t s_cur, s_next;
     __shared__ int s_ok;
 
@@ -308,18 +319,18 @@ __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB =
 
 // angle binding: the records the planner listed as angle-carrying
 __global__ void k_bind(const BPatch* __restrict__ pt, uint32_t n, const double* __restrict__ params, plan::KOp* ops,
-                       plan::TermRec* terms)
+                       BTerm* terms)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BPatch p = pt[i];
         const double ang = p.theta0 + p.coeff * params[p.param];
+        double s, c;
+        sincos(p.kind == 0 ? ang / 2.0 : ang, &s, &c);
         if (p.kind == 0) {
-            double s, c;
-            sincos(ang / 2.0, &s, &c);
             ops[p.dst].a = c;
             ops[p.dst].b = s;
         } else {
-            terms[p.dst].theta = ang;
+            terms[p.dst].e = make_double2(c, s);
         }
     }
 }
@@ -477,7 +488,7 @@ struct qse_batch {
     const uint32_t* csr_occ = nullptr;
     const double* csr_fac = nullptr;
     qse::plan::KOp* d_ops = nullptr;
-    qse::plan::TermRec* d_terms = nullptr;
+    BTerm* d_terms = nullptr;
     double* occ = nullptr;
     double* params = nullptr;
     double* values = nullptr;
@@ -523,7 +534,7 @@ void build(qse_batch* b)
 
     std::vector<plan::KOp> ops;
     std::vector<plan::LayoutRec> layouts;
-    std::vector<plan::TermRec> terms;
+    std::vector<BTerm> terms;
     std::vector<plan::GroupRec> groups;
     std::vector<double> mats;
     std::vector<BPass> passes;
@@ -548,6 +559,7 @@ void build(qse_batch* b)
         opt.max_terms = 512;
         opt.keep_gphase = false;
         opt.direct_phases = true;
+        opt.acc_mul = true;
         opt.max_slots = cf.grad_slots;
         uint32_t perm0[64];
         for (uint32_t q = 0; q < 64; ++q) perm0[q] = q;
@@ -651,7 +663,8 @@ void build(qse_batch* b)
             }
             ops.insert(ops.end(), P.ops.begin(), P.ops.end());
             layouts.insert(layouts.end(), P.layouts.begin(), P.layouts.end());
-            terms.insert(terms.end(), P.terms.begin(), P.terms.end());
+            for (const plan::TermRec& t : P.terms)
+                terms.push_back(BTerm{make_double2(std::cos(t.theta), std::sin(t.theta)), t.ocond, 0});
             groups.insert(groups.end(), P.groups.begin(), P.groups.end());
             mats.insert(mats.end(), P.mats.begin(), P.mats.end());
             passes.push_back(bp);
@@ -789,7 +802,7 @@ void build(qse_batch* b)
     A.passes = reinterpret_cast<const BPass*>(pd + o_passes);
     A.ops = reinterpret_cast<const plan::KOp*>(pd + o_ops);
     A.layouts = reinterpret_cast<const plan::LayoutRec*>(pd + o_lay);
-    A.terms = reinterpret_cast<const plan::TermRec*>(pd + o_terms);
+    A.terms = reinterpret_cast<const BTerm*>(pd + o_terms);
     A.groups = reinterpret_cast<const plan::GroupRec*>(pd + o_groups);
     A.mats = reinterpret_cast<const double*>(pd + o_mats);
     A.circs = reinterpret_cast<const BCirc*>(pd + o_circs);
@@ -806,7 +819,7 @@ void build(qse_batch* b)
     A.max_slots = max_slots;
     A.spin_limit = b->wait_limit ? b->wait_limit : kDefaultWaitPolls;
     b->d_ops = reinterpret_cast<plan::KOp*>(pd + o_ops);
-    b->d_terms = reinterpret_cast<plan::TermRec*>(pd + o_terms);
+    b->d_terms = reinterpret_cast<BTerm*>(pd + o_terms);
     b->patches = reinterpret_cast<const BPatch*>(pd + o_pt);
     b->npatches = uint32_t(patches.size());
     b->fins = reinterpret_cast<const FinPass*>(pd + o_fin);

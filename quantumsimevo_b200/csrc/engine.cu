@@ -386,7 +386,7 @@ constexpr uint32_t kLowLanesQubits = 23;
 
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
-// compiling, for the interpreter (angle accumulators, use_jit = false).
+// compiling, for the interpreter (use_jit = false).
 // Plans are kept in the context's plan cache.
 std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>& gates, plan::Options opt, int ns,
                                     bool prob_out = false)
@@ -394,7 +394,8 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     qse_ctx* ctx = st->ctx;
     auto e = std::make_shared<PlanEntry>();
     e->use_jit = ctx->jit != 0;
-    opt.acc_mul = opt.unit_rot = e->use_jit;
+    opt.acc_mul = true;
+    opt.unit_rot = e->use_jit;
     KeyWriter w;
     w.put('F');
     w.put(ctx->jit);
@@ -440,7 +441,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
         if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > (opt.rb <= 3 ? kJitMaxNewSmall : kJitMaxNewKernels)) {
             e->use_jit = false;
             e->srcs.clear();
-            opt.acc_mul = opt.unit_rot = false;
+            opt.unit_rot = false;
             opt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
             if (ns == 1) opt.k = tile_qubits_for(ctx, st->n, 4, 12);
             e->opt = opt;

@@ -11,9 +11,9 @@
 // 16-byte accesses on distinct bank groups.
 //
 // Diagonal gates never move data.  Their phase terms are summed per CTA in a
-// prologue (terms whose outer bits are not all set drop out) and applied per
-// thread as accumulated angles (one sincos per flush) or, for terms on two or
-// more register bits, as a direct multiply.
+// prologue (terms whose outer bits are not all set drop out), turned into unit
+// phases there, and applied per thread as accumulated products or, for terms on
+// two or more register bits, as a direct multiply.
 //
 // NS == 2 runs the adjoint sweep: the same gates are applied to |psi> and
 // |lambda>, and K_GRAD_* ops reduce 2 Im<lambda|G|psi> for the generator G of
@@ -36,15 +36,15 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
     const uint32_t tsize = 1u << A.k;
     double2* xbuf = smem;
     double2* gval = smem + tsize;
-    double* acc = reinterpret_cast<double*>(gval + A.ngroups);
-    double* wpart = acc + RB * blockDim.x;
+    double2* acc = gval + A.ngroups;
+    double* wpart = reinterpret_cast<double*>(acc + RB * blockDim.x);
     const uint32_t nwarps = (blockDim.x + 31) >> 5;
-    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = 0.0;
+    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = make_double2(1.0, 0.0);
 
     const uint64_t obase = tile_base(blockIdx.x, A.outer_mask);
     group_values(A.groups, A.ngroups, A.terms, obase, gval);
     if (NS == 2)
-        for (uint32_t i = tid; i < A.nslots * nwarps; i += blockDim.x) wpart[i] = 0.0;
+        for (uint32_t i = tid; i < A.nslots * wpart_stride(nwarps); i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const plan::LayoutRec* lay = A.layouts + A.layout0;
@@ -72,11 +72,8 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
     }
     if (NS == 2) {
         __syncthreads();
-        for (uint32_t s = tid; s < A.nslots; s += blockDim.x) {
-            double v = 0.0;
-            for (uint32_t w = 0; w < nwarps; ++w) v += wpart[s * nwarps + w];
-            A.slot_partial[uint64_t(s) * gridDim.x + blockIdx.x] = v;
-        }
+        for (uint32_t s = tid; s < A.nslots; s += blockDim.x)
+            A.slot_partial[uint64_t(s) * gridDim.x + blockIdx.x] = slot_sum(wpart + s * wpart_stride(nwarps), nwarps);
     }
 }
 
@@ -127,8 +124,8 @@ void pass_timer_end(qse_ctx* ctx, cudaEvent_t stop)
 size_t pass_smem_bytes(uint32_t k, uint32_t ngroups, uint32_t nslots, uint32_t rb, int nstates)
 {
     size_t threads = size_t(1) << (k - rb);
-    size_t b = (size_t(1) << k) * 16 + size_t(ngroups) * 16 + size_t(rb) * threads * 8;
-    if (nstates == 2) b += size_t(nslots) * ((threads + 31) / 32) * 8;
+    size_t b = (size_t(1) << k) * 16 + size_t(ngroups) * 16 + size_t(rb) * threads * 16;
+    if (nstates == 2) b += size_t(nslots) * dev::wpart_stride(uint32_t((threads + 31) / 32)) * 8;
     return b;
 }
 

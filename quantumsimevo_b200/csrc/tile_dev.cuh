@@ -232,16 +232,16 @@ __device__ __forceinline__ uint32_t sidx(uint32_t sb, const uint32_t (&sreg)[RB]
     return s;
 }
 
-// acc: the thread's accumulated angle of register bit p (shared memory)
+__device__ __forceinline__ bool is_one(double2 e) { return e.x == 1.0 && e.y == 0.0; }
+
+// acc: the thread's accumulated phase of register bit p (shared memory)
 template <int RB, int NS>
-__device__ __forceinline__ void flush_reg(int p, double* acc, double2 (&a)[NS][1 << RB], int nact)
+__device__ __forceinline__ void flush_reg(int p, double2* acc, double2 (&a)[NS][1 << RB], int nact)
 {
-    const double v = *acc;
-    if (v != 0.0) {
-        *acc = 0.0;
-        double s, c;
-        sincos(v, &s, &c);
-        OpPhase1 ph{make_double2(c, s)};
+    const double2 v = *acc;
+    if (!is_one(v)) {
+        *acc = make_double2(1.0, 0.0);
+        OpPhase1 ph{v};
 #pragma unroll
         for (int st = 0; st < NS; ++st)
             if (st < nact) pairs<RB>(p, a[st], ph);
@@ -261,9 +261,8 @@ __device__ __forceinline__ uint64_t tile_base(uint64_t c, uint64_t outer_mask)
     return obase;
 }
 
-// Per-CTA value of every diagonal group of a pass: the sum of the angles of
-// its terms whose outer condition holds for this tile, in term order; direct
-// groups store (cos, sin) of the sum, accumulator groups the sum itself.
+// Per-CTA value of every diagonal group of a pass: (cos, sin) of the sum of the
+// angles of its terms whose outer condition holds for this tile, in term order.
 __device__ __forceinline__ void group_values(const plan::GroupRec* __restrict__ groups, uint32_t ngroups,
                                              const plan::TermRec* __restrict__ terms, uint64_t obase, double2* gval)
 {
@@ -274,13 +273,9 @@ __device__ __forceinline__ void group_values(const plan::GroupRec* __restrict__ 
             const plan::TermRec t = terms[gr.first + i];
             if ((obase & t.ocond) == t.ocond) th += t.theta;
         }
-        if (gr.direct) {
-            double s, c;
-            sincos(th, &s, &c);
-            gval[g] = make_double2(c, s);
-        } else {
-            gval[g] = make_double2(th, 0.0);
-        }
+        double s, c;
+        sincos(th, &s, &c);
+        gval[g] = make_double2(c, s);
     }
 }
 
@@ -292,11 +287,34 @@ struct OpsEnv {
     const double* mats;               // K_U matrix indices are relative to this
     uint64_t obase;
     double2* xbuf;                    // 2^k slots
-    const double2* gval;              // group values of this CTA
-    double* wpart;                    // [slot][warp] gradient partials (NS == 2)
+    const double2* gval;              // group values of this CTA: unit phases
+    double* wpart;                    // gradient partials (NS == 2), wpart_stride(nwarps) per slot
     uint32_t nwarps;
-    double* acc;                      // angle accumulators, [register bit][thread] (zero on entry and exit)
+    double2* acc;                     // phase accumulators, [register bit][thread] (1 on entry and exit)
 };
+
+// Gradient partials of a slot: eight per warp (add_partial), and one double of
+// padding so that the threads that sum a slot each (slot_sum) hit distinct banks.
+__host__ __device__ constexpr uint32_t wpart_stride(uint32_t nwarps) { return 8 * nwarps + 1; }
+
+// Adds a gate's per-thread sums to its slot: two exchange steps leave eight sums a
+// warp, and the rest waits for the end of the tile, where all slots are summed at
+// once (five dependent steps per gate were a tenth of a reverse tile's latency).
+__device__ __forceinline__ void add_partial(double v, double* slot)
+{
+    const uint32_t nb = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+    const unsigned mask = nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u);
+#pragma unroll
+    for (int o = 16; o >= 8; o >>= 1)
+        if (uint32_t(o) < nb) v += __shfl_xor_sync(mask, v, o);
+    if (lane < 8) slot[(tid >> 5) * 8 + lane] += v;
+}
+__device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps)
+{
+    double v = 0.0;
+    for (uint32_t i = 0; i < 8 * nwarps; ++i) v += slot[i];
+    return v;
+}
 
 // Executes a pass program on the registers a[NS][R], which hold layout `lay` and
 // leave in the layout returned.  nact states take part
@@ -310,9 +328,8 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
 {
     constexpr int R = 1 << RB;
     const uint32_t tid = threadIdx.x;
-    const uint32_t warp = tid >> 5, lane = tid & 31;
-    double acc_thr = 0.0;
-    double* const acc = E.acc + tid;
+    double2 acc_thr = make_double2(1.0, 0.0);
+    double2* const acc = E.acc + tid;
 
     KOp nxt = E.nops ? E.ops[0] : KOp{};
     for (uint32_t i = 0; i < E.nops; ++i) {
@@ -371,10 +388,10 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
             break;
         }
         case plan::K_ACC_THR:
-            if (tc) acc_thr += E.gval[op.g].x;
+            if (tc) acc_thr = cmul(acc_thr, E.gval[op.g]);
             break;
         case plan::K_ACC_REG: {
-            if (tc) acc[op.p * blockDim.x] += E.gval[op.g].x;
+            if (tc) acc[op.p * blockDim.x] = cmul(acc[op.p * blockDim.x], E.gval[op.g]);
             break;
         }
         case plan::K_PHD: {
@@ -393,14 +410,9 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
 #pragma unroll
             for (int r = 0; r < RB; ++r)
                 if ((op.f >> r) & 1) flush_reg<RB, NS>(r, acc + r * blockDim.x, a, nact);
-            double2 e = make_double2(op.a, op.b);
-            if (acc_thr != 0.0) {
-                double s, c;
-                sincos(acc_thr, &s, &c);
-                e = cmul(e, make_double2(c, s));
-                acc_thr = 0.0;
-            }
-            if (e.x != 1.0 || e.y != 0.0) {
+            const double2 e = cmul(make_double2(op.a, op.b), acc_thr);
+            acc_thr = make_double2(1.0, 0.0);
+            if (!is_one(e)) {
 #pragma unroll
                 for (int st = 0; st < NS; ++st)
                     if (st < nact)
@@ -460,8 +472,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
                             if ((j & op.f) == op.f) part += im_ls(a[1][j], a[0][j]);
                     }
                 }
-                part = warp_sum(part * op.a);
-                if (lane == 0) E.wpart[op.g * E.nwarps + warp] += part;
+                add_partial(part * op.a, E.wpart + op.g * wpart_stride(E.nwarps));
             }
             break;
         }
