@@ -43,7 +43,7 @@ enum KKind : uint8_t {
     K_KIND_COUNT
 };
 
-struct KOp {
+struct alignas(16) KOp {
     uint8_t kind;
     uint8_t p;
     uint8_t q;

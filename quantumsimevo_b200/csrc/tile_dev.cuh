@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "planner.h"
 
 namespace qse {
@@ -22,9 +24,8 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// Im(conj(l) * s), Re(conj(l) * s)
+// Im(conj(l) * s)
 __device__ __forceinline__ double im_ls(double2 l, double2 s) { return l.x * s.y - l.y * s.x; }
-__device__ __forceinline__ double re_ls(double2 l, double2 s) { return l.x * s.x + l.y * s.y; }
 
 template <int R, int P, class F>
 __device__ __forceinline__ void pairs_at(double2 (&a)[R], F& f)
@@ -316,6 +317,29 @@ __device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps)
     return v;
 }
 
+// A program record as two 16-byte words, its fields taken out where they are used
+// (loaded field by field, a record is eight loads).
+struct OpWords {
+    uint4 h, v;
+    __device__ __forceinline__ void load(const KOp* op)
+    {
+        const uint4* p = reinterpret_cast<const uint4*>(op);
+        h = __ldg(p);
+        v = __ldg(p + 1);
+    }
+    __device__ __forceinline__ uint32_t kind() const { return h.x & 0xffu; }
+    __device__ __forceinline__ int p() const { return int((h.x >> 8) & 0xffu); }
+    __device__ __forceinline__ int f() const { return int(h.x >> 24); }
+    __device__ __forceinline__ uint32_t tcond() const { return h.y & 0xffffu; }
+    __device__ __forceinline__ uint32_t g() const { return h.y >> 16; }
+    __device__ __forceinline__ uint64_t ocond() const { return uint64_t(h.z) | uint64_t(h.w) << 32; }
+    __device__ __forceinline__ double a() const { return __hiloint2double(int(v.y), int(v.x)); }
+    __device__ __forceinline__ double b() const { return __hiloint2double(int(v.w), int(v.z)); }
+};
+static_assert(offsetof(KOp, kind) == 0 && offsetof(KOp, p) == 1 && offsetof(KOp, f) == 3 && offsetof(KOp, tcond) == 4 &&
+                  offsetof(KOp, g) == 6 && offsetof(KOp, ocond) == 8 && offsetof(KOp, a) == 16 && alignof(KOp) == 16,
+              "OpWords reads KOp");
+
 // Executes a pass program on the registers a[NS][R], which hold layout `lay` and
 // leave in the layout returned.  nact states take part
 // (1: only |psi>, forward; NS: the adjoint sweep on |psi> and |lambda>).
@@ -331,86 +355,87 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
     double2 acc_thr = make_double2(1.0, 0.0);
     double2* const acc = E.acc + tid;
 
-    KOp nxt = E.nops ? E.ops[0] : KOp{};
+    OpWords nxt;
+    if (E.nops) nxt.load(E.ops);
     for (uint32_t i = 0; i < E.nops; ++i) {
-        const KOp op = nxt;
-        if (i + 1 < E.nops) nxt = E.ops[i + 1];  // in flight while this op executes
-        const bool tc = (tid & op.tcond) == op.tcond;
-        switch (op.kind) {
+        const OpWords op = nxt;
+        nxt.load(E.ops + min(i + 1, E.nops - 1));  // in flight while this op executes
+        const bool tc = (tid & op.tcond()) == op.tcond();
+        switch (op.kind()) {
         case plan::K_H: {
             OpH f;
 #pragma unroll
             for (int st = 0; st < NS; ++st)
-                if (st < nact) pairs<RB>(op.p, a[st], f);
+                if (st < nact) pairs<RB>(op.p(), a[st], f);
             break;
         }
         case plan::K_X: {
-            if (tc && (E.obase & op.ocond) == op.ocond) {
-                OpX f{op.f};
+            if (tc && (E.obase & op.ocond()) == op.ocond()) {
+                OpX f{op.f()};
 #pragma unroll
                 for (int st = 0; st < NS; ++st)
-                    if (st < nact) pairs<RB>(op.p, a[st], f);
+                    if (st < nact) pairs<RB>(op.p(), a[st], f);
             }
             break;
         }
         case plan::K_Y: {
-            if (tc && (E.obase & op.ocond) == op.ocond) {
-                OpY f{op.f};
+            if (tc && (E.obase & op.ocond()) == op.ocond()) {
+                OpY f{op.f()};
 #pragma unroll
                 for (int st = 0; st < NS; ++st)
-                    if (st < nact) pairs<RB>(op.p, a[st], f);
+                    if (st < nact) pairs<RB>(op.p(), a[st], f);
             }
             break;
         }
         case plan::K_RX: {
-            OpRX f{op.a, op.b};
+            OpRX f{op.a(), op.b()};
 #pragma unroll
             for (int st = 0; st < NS; ++st)
-                if (st < nact) pairs<RB>(op.p, a[st], f);
+                if (st < nact) pairs<RB>(op.p(), a[st], f);
             break;
         }
         case plan::K_RY: {
-            OpRY f{op.a, op.b};
+            OpRY f{op.a(), op.b()};
 #pragma unroll
             for (int st = 0; st < NS; ++st)
-                if (st < nact) pairs<RB>(op.p, a[st], f);
+                if (st < nact) pairs<RB>(op.p(), a[st], f);
             break;
         }
         case plan::K_U: {
-            if (tc && (E.obase & op.ocond) == op.ocond) {
-                const double* m = E.mats + 8 * op.g;
+            if (tc && (E.obase & op.ocond()) == op.ocond()) {
+                const double* m = E.mats + 8 * op.g();
                 OpU f{make_double2(m[0], m[1]), make_double2(m[2], m[3]), make_double2(m[4], m[5]),
-                      make_double2(m[6], m[7]), op.f};
+                      make_double2(m[6], m[7]), op.f()};
 #pragma unroll
                 for (int st = 0; st < NS; ++st)
-                    if (st < nact) pairs<RB>(op.p, a[st], f);
+                    if (st < nact) pairs<RB>(op.p(), a[st], f);
             }
             break;
         }
         case plan::K_ACC_THR:
-            if (tc) acc_thr = cmul(acc_thr, E.gval[op.g]);
+            if (tc) acc_thr = cmul(acc_thr, E.gval[op.g()]);
             break;
         case plan::K_ACC_REG: {
-            if (tc) acc[op.p * blockDim.x] = cmul(acc[op.p * blockDim.x], E.gval[op.g]);
+            if (tc) acc[op.p() * blockDim.x] = cmul(acc[op.p() * blockDim.x], E.gval[op.g()]);
             break;
         }
         case plan::K_PHD: {
             if (tc) {
-                double2 e = E.gval[op.g];
+                double2 e = E.gval[op.g()];
 #pragma unroll
                 for (int st = 0; st < NS; ++st)
-                    if (st < nact) phase_masked<RB>(op.f, a[st], e);
+                    if (st < nact) phase_masked<RB>(op.f(), a[st], e);
             }
             break;
         }
         case plan::K_FLUSH_REG:
-            flush_reg<RB, NS>(op.p, acc + op.p * blockDim.x, a, nact);
+            flush_reg<RB, NS>(op.p(), acc + op.p() * blockDim.x, a, nact);
             break;
         case plan::K_FLUSH_ALL: {
 #pragma unroll
             for (int r = 0; r < RB; ++r)
-                if ((op.f >> r) & 1) flush_reg<RB, NS>(r, acc + r * blockDim.x, a, nact);
-            const double2 e = cmul(make_double2(op.a, op.b), acc_thr);
+                if ((op.f() >> r) & 1) flush_reg<RB, NS>(r, acc + r * blockDim.x, a, nact);
+            const double2 e = cmul(make_double2(op.a(), op.b()), acc_thr);
             acc_thr = make_double2(1.0, 0.0);
             if (!is_one(e)) {
 #pragma unroll
@@ -422,7 +447,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
             break;
         }
         case plan::K_TRANSPOSE: {
-            lay = E.layouts + op.g;
+            lay = E.layouts + op.g();
             const uint32_t sbw = slot_of(lay->wthr, tid), sbr = slot_of(lay->rthr, tid);
             uint32_t sreg_w[RB], sreg_r[RB];
 #pragma unroll
@@ -450,29 +475,47 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
         case plan::K_GRAD_Z:
         case plan::K_GRAD_P: {
             if constexpr (NS == 2) {
-                double part = 0.0;
-                if (op.kind == plan::K_GRAD_X || op.kind == plan::K_GRAD_Y) {
-                    const bool isx = op.kind == plan::K_GRAD_X;
+                // each a branch of its own with four chains of FMAs: a kind or a
+                // register sign decided per amplitude took three times the
+                // instructions of the sums
+                double part = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0, c3 = 0.0;
+                if (op.kind() == plan::K_GRAD_X) {
                     auto f = [&](const double2& s0, const double2& s1, const double2& l0, const double2& l1) {
-                        part += isx ? (im_ls(l0, s1) + im_ls(l1, s0)) : (re_ls(l1, s0) - re_ls(l0, s1));
+                        c0 = fma(l0.x, s1.y, c0);
+                        c1 = fma(-l0.y, s1.x, c1);
+                        c2 = fma(l1.x, s0.y, c2);
+                        c3 = fma(-l1.y, s0.x, c3);
                     };
-                    pairs2<RB>(op.p, a[0], a[NS - 1], f);
-                } else if (op.kind == plan::K_GRAD_Z) {
-                    double sg = ((tid & op.tcond) != 0) != ((E.obase & op.ocond) != 0) ? -1.0 : 1.0;
-#pragma unroll
-                    for (int j = 0; j < R; ++j) {
-                        double v = im_ls(a[1][j], a[0][j]);
-                        part += (op.p < RB && ((j >> op.p) & 1)) ? -v : v;
-                    }
-                    part *= sg;
+                    pairs2<RB>(op.p(), a[0], a[NS - 1], f);
+                    part = (c0 + c1) + (c2 + c3);
+                } else if (op.kind() == plan::K_GRAD_Y) {
+                    auto f = [&](const double2& s0, const double2& s1, const double2& l0, const double2& l1) {
+                        c0 = fma(l1.x, s0.x, c0);
+                        c1 = fma(l1.y, s0.y, c1);
+                        c2 = fma(-l0.x, s1.x, c2);
+                        c3 = fma(-l0.y, s1.y, c3);
+                    };
+                    pairs2<RB>(op.p(), a[0], a[NS - 1], f);
+                    part = (c0 + c1) + (c2 + c3);
+                } else if (op.kind() == plan::K_GRAD_Z) {
+                    const bool reg = op.p() < RB;   // else the sign is the thread's or the CTA's
+                    auto f = [&](const double2& s0, const double2& s1, const double2& l0, const double2& l1) {
+                        c0 = fma(l0.x, s0.y, c0);
+                        c1 = fma(-l0.y, s0.x, c1);
+                        c2 = fma(l1.x, s1.y, c2);
+                        c3 = fma(-l1.y, s1.x, c3);
+                    };
+                    pairs2<RB>(reg ? op.p() : 0, a[0], a[NS - 1], f);
+                    part = reg ? (c0 + c1) - (c2 + c3) : (c0 + c1) + (c2 + c3);
+                    if (((tid & op.tcond()) != 0) != ((E.obase & op.ocond()) != 0)) part = -part;
                 } else {
-                    if (tc && (E.obase & op.ocond) == op.ocond) {
+                    if (tc && (E.obase & op.ocond()) == op.ocond()) {
 #pragma unroll
                         for (int j = 0; j < R; ++j)
-                            if ((j & op.f) == op.f) part += im_ls(a[1][j], a[0][j]);
+                            if ((j & op.f()) == op.f()) part += im_ls(a[1][j], a[0][j]);
                     }
                 }
-                add_partial(part * op.a, E.wpart + op.g * wpart_stride(E.nwarps));
+                add_partial(part * op.a(), E.wpart + op.g() * wpart_stride(E.nwarps));
             }
             break;
         }
