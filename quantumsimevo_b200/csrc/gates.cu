@@ -237,36 +237,54 @@ __global__ void __launch_bounds__(kBlock) k_swap(double2* __restrict__ a, uint64
 // least (n >= 10), so reads and writes run over whole 512-byte pieces; the slot
 // of tile index r folds S's partner bits into the low three so that both sides
 // touch eight distinct 16-byte bank groups per quarter-warp.  Bound by HBM: 32 B
-// per amplitude.  The 15 pairs of a 30-qubit QFT's reversal take 5.7 ms (6.0 TB/s);
+// per amplitude.  The 15 pairs of a 30-qubit QFT's reversal take 5.5 ms (6.3 TB/s);
 // one k_swap per pair (half a sweep each) took 53 ms.
-constexpr uint32_t kInvBits = 11;   // largest tile: two of them are 64 KiB, three CTAs per SM
+//
+// Only tile pairs are launched: with k exchanged pairs among the outer bits, the
+// first of them whose bits differ is given the values (1, 0) (the partner tile
+// has (0, 1)), the pairs before it equal bits, the others every value; the last
+// segment has all pairs equal, its tiles their own partners.  (One CTA per tile,
+// half of which leave at once, took 7.5 ms at 30 qubits.)
+// Tiles of 2^12 (two of them 128 KiB, one CTA of 512 threads per SM) took 6.5 ms
+// there, and 0.79 instead of 0.66 ms at 27 qubits.
+constexpr uint32_t kInvBits = 11;      // largest tile: two of them are 64 KiB, three CTAs per SM
+constexpr uint32_t kInvThreads = 256;
 struct InvPlan {
-    uint64_t outer_mask;          // physical bits outside S
     uint32_t s;                   // tile bits
+    uint32_t npairs, nfixed;      // outer bits: exchanged pairs and bits that stay
+    uint8_t pair_lo[32], pair_hi[32], fixed[64];
     uint8_t partner[64];          // t
     uint8_t sphys[kInvBits + 1];  // S ascending
     uint16_t img[kInvBits + 1];   // slot image of tile bit b
     uint16_t wimg[kInvBits + 1];  // slot image of the source of write-order bit b
-    uint64_t poff[8];             // physical offset of tile index 256 j
+    uint64_t poff[8];             // physical offset of tile index kInvThreads j
     uint16_t sj[8], wj[8];        // its slot images
 };
 
 template <int EPT>
-__global__ void __launch_bounds__(kBlock) k_bit_involution(double2* __restrict__ a, const __grid_constant__ InvPlan g)
+__global__ void __launch_bounds__(kInvThreads) k_bit_involution(double2* __restrict__ a, const __grid_constant__ InvPlan g)
 {
     extern __shared__ double2 tile[];   // own tile | partner tile
     const uint32_t tid = threadIdx.x;
     uint64_t o = 0, p = 0;
     {
+        // the segment of blockIdx.x: the first pair that differs (npairs: none)
         uint64_t c = blockIdx.x;
-        for (uint64_t m = g.outer_mask; m; m &= m - 1, c >>= 1)
-            if (c & 1) {
-                const uint32_t b = __ffsll(static_cast<long long>(m)) - 1;
-                o |= uint64_t(1) << b;
-                p |= uint64_t(1) << g.partner[b];
-            }
+        uint32_t d = 0;
+        for (uint64_t len = uint64_t(1) << (2 * g.npairs + g.nfixed) >> 2; d < g.npairs && c >= len; ++d, len >>= 1) c -= len;
+        auto take = [&] {
+            const uint64_t b = c & 1;
+            c >>= 1;
+            return b;
+        };
+        for (uint32_t i = 0; i < g.nfixed; ++i) o |= take() << g.fixed[i];
+        p = o;
+        for (uint32_t i = 0; i < g.npairs; ++i) {
+            const uint64_t lo = i == d ? 1 : take(), hi = i < d ? lo : i == d ? 0 : take();
+            o |= lo << g.pair_lo[i] | hi << g.pair_hi[i];
+            p |= hi << g.pair_lo[i] | lo << g.pair_hi[i];
+        }
     }
-    if (p < o) return;   // the partner's CTA does both
     const bool self = p == o;
     double2* const other = tile + (self ? 0u : 1u << g.s);
     uint64_t t = 0;
@@ -519,7 +537,6 @@ void launch_bit_involution(qse_state* st, const uint32_t* partner)
     InvPlan g{};
     uint64_t S = 0;
     for (uint32_t b = 0; b < n; ++b) {
-        g.partner[b] = uint8_t(partner[b]);
         const uint64_t add = (uint64_t(1) << b) | (uint64_t(1) << partner[b]);
         if (uint32_t(__builtin_popcountll(S | add)) <= kInvBits) S |= add;
     }
@@ -529,7 +546,14 @@ void launch_bit_involution(qse_state* st, const uint32_t* partner)
             rank[b] = g.s;
             g.sphys[g.s++] = uint8_t(b);
         }
-    g.outer_mask = ((uint64_t(1) << n) - 1) & ~S;
+    for (uint32_t b = 0; b < n; ++b) {
+        if ((S >> b) & 1) continue;
+        if (partner[b] == b) g.fixed[g.nfixed++] = uint8_t(b);
+        else if (partner[b] > b) {
+            g.pair_lo[g.npairs] = uint8_t(b);
+            g.pair_hi[g.npairs++] = uint8_t(partner[b]);
+        }
+    }
     // tile bit i of the write order reads tile bit src[i].  The lanes of a
     // quarter-warp vary tile bits 0..2 on the store side and src[0..2] on the
     // load side: a source at 3 or above takes a low image that the others leave
@@ -561,8 +585,10 @@ void launch_bit_involution(qse_state* st, const uint32_t* partner)
     QSE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     double2* a = reinterpret_cast<double2*>(st->amp);
     void* args[] = {&a, &g};
-    QSE_CUDA(cudaLaunchKernel(k, dim3(unsigned(st->size() >> g.s)), dim3(std::min(256u, 1u << g.s)), args, smem,
-                              st->ctx->stream));
+    // tiles that are their own partners, and half of the others
+    const uint64_t tiles = st->size() >> g.s, own = uint64_t(1) << (g.npairs + g.nfixed);
+    QSE_CUDA(cudaLaunchKernel(k, dim3(unsigned(own + (tiles - own) / 2)), dim3(std::min(kInvThreads, 1u << g.s)), args,
+                              smem, st->ctx->stream));
     count_launch(st->ctx);
 }
 }  // namespace
