@@ -85,7 +85,7 @@ struct KeyWriter {
     void put_options(const plan::Options& o)
     {
         put(o.k); put(o.rb); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
-        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.keep_gphase);
+        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.lane_swaps); put(o.keep_gphase);
     }
     // everything but the angles and the matrices
     void put_gates(const std::vector<plan::Gate>& gates)
@@ -383,6 +383,13 @@ constexpr uint32_t kSmallQubits = 20;
 // 26-qubit H+RZ+QFT 0.74 -> 0.75 ms.  At 22 qubits the exchanges cost more than
 // the accesses (HEA gradient 1.84 -> 1.91 ms).
 constexpr uint32_t kLowLanesQubits = 23;
+// States of at least this many qubits move what is left of the lowest qubits to
+// the lanes by shuffles (Options::lane_swaps).  On top of low_lanes: 28-qubit
+// QAOA energy 8.1 -> 7.6 ms, 24-qubit gradients of a HEA 4.5 -> 4.1 ms and of a
+// QAOA circuit 4.4 -> 4.1 ms; alone (without low_lanes the 28-qubit energy takes
+// 8.5 ms): 22-qubit HEA gradient 1.74 -> 1.69 ms, 20 qubits 0.74 -> 0.72 ms; no
+// gain below.
+constexpr uint32_t kLaneSwapQubits = 20;
 
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
@@ -584,6 +591,7 @@ plan::Options fused_options(const qse_ctx* ctx, uint32_t n)
     if (ctx->jit && (opt.max_gates == 0 || opt.max_gates > plan::kJitMaxGates)) opt.max_gates = plan::kJitMaxGates;
     opt.zz_fuse = true;
     opt.low_lanes = n >= kLowLanesQubits;
+    opt.lane_swaps = n >= kLaneSwapQubits;
     return opt;
 }
 
@@ -1364,6 +1372,7 @@ double adjoint_sweep(qse_state* st, const qse_op* ops, size_t nops, const double
     opt.max_terms = 512;
     opt.max_gates = plan::kJitMaxGates;
     opt.low_lanes = st->n >= kLowLanesQubits;
+    opt.lane_swaps = st->n >= kLaneSwapQubits;
     const std::shared_ptr<PlanEntry> e = plan_for(st, rev, opt, 2);
     const plan::Plan& pl = e->pl;
     Uploaded up = upload_plan(ctx, pl, e->use_jit, e->use_jit && st->n >= jit::kPreGroupQubits);

@@ -201,6 +201,34 @@ struct Gen {
         }
     }
 
+    // Reading and writing memory with physical qubits 0..2 in registers leaves
+    // every lane a line of its own (or half sectors), whatever layout the gates
+    // want.  Where a pass begins or ends that way, those register bits trade
+    // places with lane bits on the memory side by shuffles inside the warp (four
+    // per two amplitudes and bit; no shared memory, no barrier): reg/thr become
+    // the memory layout, and the swaps lead from one to the other either way.
+    struct LaneSwap { uint32_t i; int t; };
+    std::vector<LaneSwap> to_memory_layout()
+    {
+        std::vector<LaneSwap> v;
+        if (!P.lane_swaps || T < 32) return v;
+        int t = 4;
+        for (uint32_t i = 0; i < P.rb; ++i) {
+            if (P.tile_phys[reg[i]] >= 3) continue;
+            while (t >= 0 && P.tile_phys[thr[t]] < 3) --t;
+            if (t < 0) break;
+            std::swap(reg[i], thr[t]);
+            v.push_back({i, t--});
+        }
+        return v;
+    }
+    void emit_swaps(const std::vector<LaneSwap>& v)
+    {
+        for (const LaneSwap& s : v)
+            for (int st = 0; st < ns; ++st)
+                o << "  laneSwap<" << s.i << ", " << s.t << ">(a" << st << ");\n";
+    }
+
     static std::string hex(uint64_t v)
     {
         char b[32];
@@ -556,7 +584,9 @@ struct Gen {
         if (!P.acc_mul) emit_acc_decls();
         for (const plan::KOp& op : P.ops) emit_op(op);
         flush_run();
-        // store (final layout)
+        // store (final layout, its lowest qubits moved to the lanes)
+        emit_swaps(to_memory_layout());
+        o << "  gb = " << gbase_expr() << ";\n";
         for (uint32_t j = 0; j < R; ++j) {
             const std::string ix = "gb + " + hex(reg_off(j));
             o << "  " << guard(ix, nstr()) << "psi[" << ix << "] = a0[" << j << "];";
@@ -622,6 +652,7 @@ struct Gen {
         // load first (gb holds only thread and outer bits, the offsets only
         // register bits: gb + off == gb | off, and the constant folds into the
         // address); the prologue below then runs while the loads are in flight
+        const std::vector<LaneSwap> in_swaps = zero_in ? std::vector<LaneSwap>() : to_memory_layout();
         o << "  u64 gb = " << gbase_expr() << ";\n";
         for (int s = 0; s < ns; ++s) o << "  double2 a" << s << "[" << R << "];\n";
         if (!zero_in) {
@@ -740,6 +771,7 @@ struct Gen {
             o << "    pfs[j] = f;\n  }\n";
         }
         o << "  __syncthreads();\n";
+        emit_swaps(in_swaps);
         if (zero_in && !umask)
             for (uint32_t j = 0; j < R; ++j)
                 o << "  a0[" << j << "] = make_double2((gb | " << hex(reg_off(j)) << ") == bi ? 1.0 : 0.0, 0.0);\n";
@@ -971,6 +1003,7 @@ struct Gen {
         if (!P.acc_mul) emit_acc_decls();
         for (const plan::KOp& op : P.ops) emit_op(op);
         flush_run();
+        o << "      gb = " << gbase_expr() << ";\n";
         for (uint32_t j = 0; j < R; ++j) o << "      psi[gb + " << hex(reg_off(j)) << "] = a0[" << j << "];\n";
         std::swap(o, body);
         const std::string ops_txt = body.str();
@@ -1168,7 +1201,7 @@ struct Gen {
                 for (uint32_t j = 0; j < R; ++j)
                     o << "    " << A << "[" << j << "] = xb[sr ^ " << slot_off(nl, j) << "u];\n";
             }
-            o << "    gb = " << gbase_expr() << ";\n  }\n";
+            o << "  }\n";
             break;
         }
         case K_GRAD_X: case K_GRAD_Y:

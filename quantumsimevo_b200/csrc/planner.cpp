@@ -770,6 +770,7 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         prog.k = k;
         prog.rb = opt.rb;
         prog.acc_mul = opt.acc_mul;
+        prog.lane_swaps = opt.lane_swaps;
         uint32_t b = 0;
         for (uint32_t q = 0; q < n; ++q)
             if ((T >> q) & 1) prog.tile_phys[b++] = uint8_t(q);

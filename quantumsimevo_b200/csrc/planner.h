@@ -99,6 +99,7 @@ struct PassProgram {
     uint32_t k = 0;                 // tile qubits
     uint32_t rb = 4;                // register bits per thread
     bool acc_mul = false;           // accumulators carry complex factors (Options::acc_mul)
+    bool lane_swaps = false;        // Options::lane_swaps
     uint64_t outer_mask = 0;        // physical qubits not in the tile
     uint8_t tile_phys[16] = {0};    // physical qubit of tile-local bit b (ascending)
     uint32_t layout0 = 0;           // layout at load time (index into layouts)
@@ -165,7 +166,9 @@ struct Options {
     bool zz_fuse = false;        // rewrite CNOT(c,t) RZ(th,t) CNOT(c,t) as the diagonal
                                  // RZ(th,c) PHASE(th,t) CPHASE(-2th,c,t) (same three slots;
                                  // only for plans whose angles are never rebound)
-    bool low_lanes = false;      // keep physical qubits 0..2 out of the registers where a pass reads and writes
+    bool lane_swaps = false;     // specialised kernels move physical qubits 0..2 from the registers to the
+                                 // lanes by shuffles where a pass reads and writes
+    bool low_lanes = false;      // the layouts keep physical qubits 0..2 out of the registers where a pass reads and writes
     bool unit_rot = false;       // rotations divided by their larger entry, one FMA per component instead
                                  // of a multiply and an FMA (kernels that take K_RX / K_RY in that form)
     bool keep_gphase = true;     // false: drop RZ's global phase (expectations and gradients
