@@ -604,7 +604,7 @@ int qse_plan_compile(uint32_t nqubits, const qse_op* ops, size_t nops, const dou
     for (uint32_t q = 0; q < 64; ++q) perm[q] = q;
     qse::plan::Options opt;
     opt.k = std::min<uint32_t>(tile_qubits ? tile_qubits : (nstates == 2 ? 11 : 12), nqubits);
-    opt.rb = nstates == 2 ? (opt.k == 11 ? 4 : 3) : (!streamed && opt.k == 12) ? 5 : 4;   // as the engine plans large states
+    opt.rb = nstates == 2 && opt.k != 11 ? 3 : 4;   // as the engine plans large states
     opt.grads = nstates == 2;
     opt.acc_mul = opt.unit_rot = true;
     opt.max_gates = qse::plan::kJitMaxGates;

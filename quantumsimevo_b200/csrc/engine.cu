@@ -84,7 +84,7 @@ struct KeyWriter {
     }
     void put_options(const plan::Options& o)
     {
-        put(o.k); put(o.rb); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
+        put(o.k); put(o.rb); put(o.rb_first); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
         put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.lane_swaps); put(o.keep_gphase);
     }
     // everything but the angles and the matrices
@@ -450,6 +450,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
             e->srcs.clear();
             opt.unit_rot = false;
             opt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
+            opt.rb_first = 0;
             if (ns == 1) opt.k = tile_qubits_for(ctx, st->n, 4, 12);
             e->opt = opt;
             e->pl = plan::build(gates, st->n, st->perm, opt);
@@ -574,15 +575,20 @@ void run_noise(qse_state* st, qse_noise* nz, const qse_op* ops, size_t nops, con
     QSE_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
-plan::Options fused_options(const qse_ctx* ctx, uint32_t n)
+plan::Options fused_options(const qse_ctx* ctx, uint32_t n, bool compact_input = false)
 {
     plan::Options opt;
     opt.rb = 4;
     opt.k = tile_qubits_for(ctx, n, 4, 12);
-    // specialised tile kernels on 4096-amplitude tiles hold 32 amplitudes per
-    // thread (128 threads, three CTAs per SM): twice the independent FP64 work
-    // per thread and one layout exchange per five register qubits instead of four
-    if (ctx->jit == 1 && opt.k == 12) opt.rb = 5;
+    // A pass that makes its input from a compact state writes memory but does not
+    // read it, and is bound by FP64 and its layout exchanges: 32 amplitudes per
+    // thread (128 threads, three CTAs per SM) take an exchange per five register
+    // qubits and share each phase factor among twice the amplitudes (30-qubit
+    // H+RZ+QFT 5.5 ms, with 16 per thread 6.8).  Passes that read and write
+    // memory hold 16 (256 threads, two CTAs): a third more warps to keep loads in
+    // flight, and half the code to fetch (27-qubit random layers 0.72-0.83 ms a
+    // pass, with 32 per thread 1.12-1.24).
+    if (ctx->jit == 1 && opt.k == 12 && compact_input) opt.rb_first = 5;
     if (ctx->jit == 1 && ctx->tile_qubits == 12 && n <= kSmallQubits) {
         opt.k = std::min(n <= kTile11Qubits ? 11u : 10u, n);
         opt.rb = 3;
@@ -603,7 +609,7 @@ uint64_t run_fused(qse_state* st, const std::vector<plan::Gate>& gates, bool pro
 {
     qse_ctx* ctx = st->ctx;
     prob_out = prob_out && st->size() >= 4096 && ctx->jit != 0;
-    const std::shared_ptr<PlanEntry> e = plan_for(st, gates, fused_options(ctx, st->n), 1, prob_out);
+    const std::shared_ptr<PlanEntry> e = plan_for(st, gates, fused_options(ctx, st->n, st->lazy_basis && st->lazy_umask), 1, prob_out);
     const plan::Plan& pl = e->pl;
     const bool use_jit = e->use_jit;
     const std::vector<jit::Source>& srcs = e->srcs;

@@ -768,7 +768,7 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         for (uint32_t q = 0; q < n && uint32_t(popc(T)) < k; ++q) T |= bit(q);
         PassProgram prog;
         prog.k = k;
-        prog.rb = opt.rb;
+        prog.rb = plan.passes.empty() && opt.rb_first ? opt.rb_first : opt.rb;
         prog.acc_mul = opt.acc_mul;
         prog.lane_swaps = opt.lane_swaps;
         uint32_t b = 0;

@@ -154,6 +154,7 @@ constexpr uint32_t kJitMaxGates = 256;
 struct Options {
     uint32_t k = 12;             // tile qubits (clamped to n)
     uint32_t rb = 4;             // register bits per thread (at most 5; the interpreter kernel takes 3 or 4)
+    uint32_t rb_first = 0;       // the first pass's register bits (0: rb)
     uint32_t max_gates = 0;      // 0 = no cap on non-diagonal gates per pass
     uint32_t max_terms = 1024;   // diagonal terms per pass (shared-memory group table)
     bool grads = false;          // emit K_GRAD_* for gates with grad >= 0
