@@ -263,6 +263,9 @@ __device__ void block_scan_maps(uint64_t t0, uint64_t t1, uint64_t& ex0, uint64_
 // sit in row tid), starting from the exact running sum c_in.  The values go
 // to out (if non-null), staged in the same buffer.  Returns the block's final
 // sum.  Must be called by all threads of the block.
+// kStays: the sum may stay in its binade (tried first); false where the caller
+// knows that it does not.
+template <bool kStays>
 __device__ __forceinline__ double block_exact(uint32_t cnt, double c_in, double* out, uint64_t* sh, double* stage)
 {
     __shared__ double s_c;
@@ -275,7 +278,7 @@ __device__ __forceinline__ double block_exact(uint32_t cnt, double c_in, double*
     // and a running sum that stays below 2^53 grid units.  The grid integers
     // and all their partial sums are then exact in FP64, so the scan runs on
     // doubles with no integer conversion; otherwise fall through.
-    if (cnt == uint32_t(kBS) && c > 0.0) {
+    if (kStays && cnt == uint32_t(kBS) && c > 0.0) {
         const int e = epoch_of(c);
         const Grid g = grid_of(e);
         if (g.fast) {
@@ -436,12 +439,23 @@ __device__ __forceinline__ double block_exact(uint32_t cnt, double c_in, double*
         }
         __syncthreads();
         // slots >= t are still the probabilities
-        pos = min(cnt, t + kRun);
+        pos = min(cnt, (t + kRun) & ~uint32_t(kEPT - 1));   // t's row and the next few
         if (tid == 0 && t < cnt) {
+            // a row at a time: its 16 loads are in flight together, so only the
+            // additions are a chain (0.0 in the places before t changes nothing)
             double cc = s_c;
-            for (uint32_t i = t; i < pos; ++i) {
-                cc = __dadd_rn(cc, stage[stage_slot(i)]);
-                if (out) stage[stage_slot(i)] = cc;
+            for (uint32_t r = t / kEPT; r * kEPT < pos; ++r) {
+                double* const row = stage + r * kPad;
+                double v[kEPT];
+#pragma unroll
+                for (int j = 0; j < kEPT; ++j) v[j] = r * kEPT + j >= t && r * kEPT + j < pos ? row[j] : 0.0;
+#pragma unroll
+                for (int j = 0; j < kEPT; ++j) v[j] = cc = __dadd_rn(cc, v[j]);
+                if (out) {
+#pragma unroll
+                    for (int j = 0; j < kEPT; ++j)
+                        if (r * kEPT + j >= t && r * kEPT + j < pos) row[j] = v[j];
+                }
             }
             s_c = cc;
         }
@@ -943,12 +957,14 @@ struct ChainIO {
     uint32_t pend[2] = {0, 0};             // copy in flight, per buffer
     uint32_t ph[2] = {0, 0};               // parity of its mbarrier phase
     uint32_t loaded[2] = {~0u, ~0u};       // first block the buffer holds (or will)
+    uint32_t end[2] = {0, 0};              // and the one after its last
     __device__ ChainIO(ChainShm& s, char* r, const Summ* sm) : S(s), raw(r), summ(sm) {}
     __device__ void fetch(uint32_t b, uint32_t from, uint32_t cnt)
     {
         if (threadIdx.x == 0) S.skew[b] = summ_fetch(raw + b * kSpanBuf, summ, from, cnt, &S.bar[b]);
         pend[b] = 1;
         loaded[b] = from;
+        end[b] = from + cnt;
     }
     // waits for buffer b's copy; uniform result (a copy not seen done stays pending)
     __device__ bool drain(uint32_t b)
@@ -975,8 +991,8 @@ struct ChainIO {
 // fold on the binade it actually starts in, else an exact element-by-element
 // fold) and the next span starts after it.  The fold records of a span arrive
 // in shared memory by bulk copies while the previous span is composed (two
-// buffers; a span that stopped early reloads its successor's records; records
-// already in buffer 0 for b_begin are used as they are).  A running sum of
+// buffers; a span that stopped early goes on in the same buffer; records already
+// in buffer 0 for b_begin are used as they are).  A running sum of
 // zero is on the grid of binade -1022 (spacing 2^-1074, shared by the
 // subnormals), where zero and subnormal blocks fold exactly.  False when a
 // bounded wait gave up.
@@ -987,15 +1003,11 @@ __device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32
     const uint32_t t = threadIdx.x;
     uint32_t base = b_begin, cur = 0;
     while (base < b_end) {
-        const uint32_t span = min(kSpan, b_end - base);
-        if (io.loaded[cur] != base) {   // the first span, or the previous span stopped early
-            if (!io.drain(0) || !io.drain(1)) return false;
-            io.fetch(cur, base, span);
-        }
-        const uint32_t next = base + span;
-        if (next < b_end) io.fetch(cur ^ 1, next, min(kSpan, b_end - next));
+        if (io.loaded[cur] == ~0u) io.fetch(cur, base, min(kSpan, b_end - base));   // the first span
+        const uint32_t next = io.end[cur], span = next - base;
+        if (next < b_end && io.loaded[cur ^ 1] != next) io.fetch(cur ^ 1, next, min(kSpan, b_end - next));
         if (!io.drain(cur)) return false;
-        const Summ* rec = io.rec(cur);
+        const Summ* rec = io.rec(cur) + (base - io.loaded[cur]);
         const double c = S.c;
         const int e0 = epoch_of(c);
         const uint32_t p0 = t * kChainPer;           // this thread's first position in the span
@@ -1053,7 +1065,7 @@ __device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32
         __syncthreads();   // every thread is done with rec and S.c before either changes
         if (end >= span) {
             base = next;
-            cur ^= 1;   // loaded[cur] == next: fetched above
+            cur ^= 1;   // fetched above
             continue;
         }
         // block b starts in the running sum's binade but has no fold there or leaves it
@@ -1080,11 +1092,12 @@ __device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32
             ++n_exact;
             double p[kEPT];
             load_block_prob(prob, uint64_t(b) * kBS, p, S.stage);
-            double cc = block_exact(kBS, S.c, nullptr, S.sh, S.stage);
+            double cc = block_exact<false>(kBS, S.c, nullptr, S.sh, S.stage);
             if (t == 0) S.c = cc;
         }
         __syncthreads();
         base = b + 1;
+        if (base == next) cur ^= 1;
     }
     return true;
 }
@@ -1494,7 +1507,7 @@ __global__ void __launch_bounds__(kBT) k_search_each(const double* __restrict__ 
     stage_async(stg, prob, uint64_t(b) * kBS);
     stage_wait<0>();
     __syncthreads();
-    block_exact(kBS, cin[b], cum, sh, stg);
+    block_exact<true>(kBS, cin[b], cum, sh, stg);
     __syncthreads();
     if (threadIdx.x == 0) out[s] = uint64_t(b) * kBS + lower_bound_dev(cum, kBS, s_t);
 }
@@ -1535,7 +1548,7 @@ __global__ void __launch_bounds__(kBT, kWriteCTAs) k_block_search(const double* 
         }
         __syncthreads();
         const uint32_t b = nonempty[k];
-        block_exact(kBS, cin[b], cum, sh, cur);
+        block_exact<true>(kBS, cin[b], cum, sh, cur);
         __syncthreads();
         for (uint32_t i = offset[b] + threadIdx.x; i < offset[b + 1]; i += kBT) {
             const uint32_t s = order[i];
