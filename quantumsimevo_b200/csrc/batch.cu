@@ -13,8 +13,8 @@
 // phase is dropped: <O> and the gradients do not see it.
 //
 // Work queue.  A circuit whose passes have at most chain_tiles tiles is ONE
-// item: a single CTA runs all its passes, forward and reverse, tile after tile
-// (the state stays in L2).  Wider circuits give one item per (pass, tile),
+// item, unless it alone would hold up the batch: a single CTA runs all its
+// passes, forward and reverse, tile after tile (the state stays in L2).  Wider circuits give one item per (pass, tile),
 // queued level-major (every circuit's pass 0, then every circuit's pass 1, ...),
 // so a tile's dependencies (all tiles of the circuit's previous pass) sit
 // earlier in the queue.  CTAs claim items in queue order with one atomic, and
@@ -121,7 +121,7 @@ struct BatchArgs {
     uint32_t max_groups;
     uint32_t max_slots;
     uint32_t spin_limit;
-    uint32_t pad;
+    uint32_t wlanes;             // gradient partials per warp and slot
 };
 
 constexpr uint32_t kMaxThreads = 512;
@@ -129,13 +129,13 @@ constexpr uint32_t kMaxThreads = 512;
 // gives up: about a second, far beyond any pass of a circuit that fits
 constexpr uint32_t kDefaultWaitPolls = 1u << 21;
 
-// exchange buffer | group values | phase accumulators | gradient partials | warp
-// sums
-size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb)
+// exchange buffer | group values | phase accumulators (16 amplitudes per thread:
+// with fewer they are in the thread's own memory) | gradient partials | warp sums
+size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb, uint32_t wlanes)
 {
     const size_t nwarps = threads / 32;
-    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + size_t(rb) * threads * 16 +
-           size_t(max_slots) * tile::dev::wpart_stride(uint32_t(nwarps)) * 8 + nwarps * 8;
+    return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + (rb == 4 ? size_t(rb) * threads * 16 : 0) +
+           size_t(max_slots) * tile::dev::wpart_stride(uint32_t(nwarps), wlanes) * 8 + nwarps * 8;
 }
 
 // ------------------------------------------------------------------ device
@@ -208,7 +208,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         gval[g] = v;
     }
     if (rev)
-        for (uint32_t i = tid; i < nslots * wpart_stride(nwarps); i += blockDim.x) wpart[i] = 0.0;
+        for (uint32_t i = tid; i < nslots * wpart_stride(nwarps, A.wlanes); i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const bool active = tid < (1u << (k - RB));
@@ -240,8 +240,11 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         }
     }
 
+    double2 own_acc[RB];
+    if (RB < 4)
+        for (int r = 0; r < RB; ++r) own_acc[r] = make_double2(1.0, 0.0);
     const OpsEnv E{A.ops + P.op0, P.nops, A.layouts + P.lay0, A.mats + 8 * size_t(P.mat0), obase,
-                   xbuf, gval, wpart, nwarps, acc};
+                   xbuf, gval, wpart, nwarps, A.wlanes, RB == 4 ? acc + tid : own_acc, RB == 4 ? blockDim.x : 1u};
     lay = run_ops<RB, 2>(E, lay, a, rev ? 2 : 1, active);
 
     if (!(flags & F_NOSTORE) && active) {
@@ -262,7 +265,8 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     if (rev && nslots) {
         __syncthreads();
         double* out = A.part + P.part0 + uint64_t(tile) * nslots;
-        for (uint32_t s = tid; s < nslots; s += blockDim.x) out[s] = slot_sum(wpart + s * wpart_stride(nwarps), nwarps);
+        for (uint32_t s = tid; s < nslots; s += blockDim.x)
+            out[s] = slot_sum(wpart + s * wpart_stride(nwarps, A.wlanes), nwarps, A.wlanes);
     }
 }
 
@@ -280,9 +284,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB =
     double2* xbuf = smem;
     double2* gval = smem + (size_t(1) << A.kmax);
     double2* acc = gval + A.max_groups;
-    double* wpart = reinterpret_cast<double*>(acc + RB * blockDim.x);
-    double* red = wpart + size_t(A.max_slots) * wpart_stride(nwarps);
-    for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = make_double2(1.0, 0.0);
+    double* wpart = reinterpret_cast<double*>(acc + (RB == 4 ? RB * blockDim.x : 0));
+    double* red = wpart + size_t(A.max_slots) * wpart_stride(nwarps, A.wlanes);
+    if (RB == 4)
+        for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = make_double2(1.0, 0.0);
     __shared__ uint32_t s_cur, s_next;
     __shared__ int s_ok;
 
@@ -697,7 +702,12 @@ void build(qse_batch* b)
     }
 
     // shared memory and grid
-    const size_t smem = smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb);
+    // as many gradient partials per warp as leave room for three CTAs per SM; with one
+    // a pass of thousands of slots still fits (eight would stop at some 690 of them)
+    auto smem_with = [&](uint32_t wl) { return smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, wl); };
+    uint32_t wlanes = 8;
+    while (wlanes > 1 && smem_with(wlanes) > 72 * 1024) wlanes /= 2;
+    const size_t smem = smem_with(wlanes);
     if (smem + 64 > ctx->smem_optin)
         fail(QSE_ERR_SIZE, "batch: a pass needs " + std::to_string(smem) +
                                " B of shared memory; lower max_gates or the tile size");
@@ -817,6 +827,7 @@ void build(qse_batch* b)
     A.kmax = kmax;
     A.max_groups = max_groups;
     A.max_slots = max_slots;
+    A.wlanes = wlanes;
     A.spin_limit = b->wait_limit ? b->wait_limit : kDefaultWaitPolls;
     b->d_ops = reinterpret_cast<plan::KOp*>(pd + o_ops);
     b->d_terms = reinterpret_cast<BTerm*>(pd + o_terms);

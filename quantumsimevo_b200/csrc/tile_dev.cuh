@@ -289,31 +289,39 @@ struct OpsEnv {
     uint64_t obase;
     double2* xbuf;                    // 2^k slots
     const double2* gval;              // group values of this CTA: unit phases
-    double* wpart;                    // gradient partials (NS == 2), wpart_stride(nwarps) per slot
-    uint32_t nwarps;
-    double2* acc;                     // phase accumulators, [register bit][thread] (1 on entry and exit)
+    double* wpart;                    // gradient partials (NS == 2), wpart_stride(nwarps, wlanes) per slot
+    uint32_t nwarps, wlanes;
+    double2* acc;                     // phase accumulators of register bit p at acc[p * acc_stride] (1 on entry and exit)
+    uint32_t acc_stride;
 };
 
-// Gradient partials of a slot: eight per warp (add_partial), and one double of
-// padding so that the threads that sum a slot each (slot_sum) hit distinct banks.
-__host__ __device__ constexpr uint32_t wpart_stride(uint32_t nwarps) { return 8 * nwarps + 1; }
+// Gradient partials of a slot: wlanes (8, 4, 2 or 1) per warp (add_partial), and,
+// above one, a double of padding so that the threads that sum a slot each
+// (slot_sum) hit distinct banks.  The launch takes as many as fit in shared memory.
+__host__ __device__ constexpr uint32_t wpart_stride(uint32_t nwarps, uint32_t wlanes)
+{
+    return wlanes * nwarps + (wlanes > 1 ? 1 : 0);
+}
 
-// Adds a gate's per-thread sums to its slot: two exchange steps leave eight sums a
-// warp, and the rest waits for the end of the tile, where all slots are summed at
-// once (five dependent steps per gate were a tenth of a reverse tile's latency).
-__device__ __forceinline__ void add_partial(double v, double* slot)
+// Adds a gate's per-thread sums to its slot: with wlanes 8, two exchange steps
+// leave eight sums a warp, and the rest waits for the end of the tile, where all
+// slots are summed at once (five dependent steps per gate were a tenth of a
+// reverse tile's latency).
+__device__ __forceinline__ void add_partial(double v, double* slot, uint32_t wlanes)
 {
     const uint32_t nb = blockDim.x, tid = threadIdx.x, lane = tid & 31;
     const unsigned mask = nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u);
 #pragma unroll
-    for (int o = 16; o >= 8; o >>= 1)
-        if (uint32_t(o) < nb) v += __shfl_xor_sync(mask, v, o);
-    if (lane < 8) slot[(tid >> 5) * 8 + lane] += v;
+    for (uint32_t o = 16; o >= 8; o >>= 1)
+        if (o < nb) v += __shfl_xor_sync(mask, v, o);
+    for (uint32_t o = 4; o >= wlanes; o >>= 1)   // only where the launch had to take fewer
+        if (o < nb) v += __shfl_xor_sync(mask, v, o);
+    if (lane < wlanes) slot[(tid >> 5) * wlanes + lane] += v;
 }
-__device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps)
+__device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps, uint32_t wlanes)
 {
     double v = 0.0;
-    for (uint32_t i = 0; i < 8 * nwarps; ++i) v += slot[i];
+    for (uint32_t i = 0; i < wlanes * nwarps; ++i) v += slot[i];
     return v;
 }
 
@@ -353,7 +361,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
     constexpr int R = 1 << RB;
     const uint32_t tid = threadIdx.x;
     double2 acc_thr = make_double2(1.0, 0.0);
-    double2* const acc = E.acc + tid;
+    double2* const acc = E.acc;
 
     OpWords nxt;
     if (E.nops) nxt.load(E.ops);
@@ -416,7 +424,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
             if (tc) acc_thr = cmul(acc_thr, E.gval[op.g()]);
             break;
         case plan::K_ACC_REG: {
-            if (tc) acc[op.p() * blockDim.x] = cmul(acc[op.p() * blockDim.x], E.gval[op.g()]);
+            if (tc) acc[op.p() * E.acc_stride] = cmul(acc[op.p() * E.acc_stride], E.gval[op.g()]);
             break;
         }
         case plan::K_PHD: {
@@ -429,12 +437,12 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
             break;
         }
         case plan::K_FLUSH_REG:
-            flush_reg<RB, NS>(op.p(), acc + op.p() * blockDim.x, a, nact);
+            flush_reg<RB, NS>(op.p(), acc + op.p() * E.acc_stride, a, nact);
             break;
         case plan::K_FLUSH_ALL: {
 #pragma unroll
             for (int r = 0; r < RB; ++r)
-                if ((op.f() >> r) & 1) flush_reg<RB, NS>(r, acc + r * blockDim.x, a, nact);
+                if ((op.f() >> r) & 1) flush_reg<RB, NS>(r, acc + r * E.acc_stride, a, nact);
             const double2 e = cmul(make_double2(op.a(), op.b()), acc_thr);
             acc_thr = make_double2(1.0, 0.0);
             if (!is_one(e)) {
@@ -515,7 +523,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
                             if ((j & op.f()) == op.f()) part += im_ls(a[1][j], a[0][j]);
                     }
                 }
-                add_partial(part * op.a(), E.wpart + op.g() * wpart_stride(E.nwarps));
+                add_partial(part * op.a(), E.wpart + op.g() * wpart_stride(E.nwarps, E.wlanes), E.wlanes);
             }
             break;
         }
