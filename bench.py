@@ -455,6 +455,8 @@ def main():
     if args.impl == "reference":
         run_reference_arm(args, rank)
         return
+    if not args.no_ref_gpu and _oracle_ffi().load_reference(gpu=True) is None:
+        args.no_ref_gpu = True   # that library was not built here: leave its baselines out
 
     import numpy as np
 
