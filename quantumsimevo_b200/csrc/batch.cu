@@ -121,7 +121,7 @@ struct BatchArgs {
     uint32_t max_groups;
     uint32_t max_slots;
     uint32_t spin_limit;
-    uint32_t wlanes;             // gradient partials per warp and slot
+    uint32_t pad;
 };
 
 constexpr uint32_t kMaxThreads = 512;
@@ -131,11 +131,11 @@ constexpr uint32_t kDefaultWaitPolls = 1u << 21;
 
 // exchange buffer | group values | phase accumulators (16 amplitudes per thread:
 // with fewer they are in the thread's own memory) | gradient partials | warp sums
-size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb, uint32_t wlanes)
+size_t smem_bytes(uint32_t kmax, uint32_t max_groups, uint32_t max_slots, uint32_t threads, uint32_t rb, uint32_t wl)
 {
     const size_t nwarps = threads / 32;
     return (size_t(1) << kmax) * 16 + size_t(max_groups) * 16 + (rb == 4 ? size_t(rb) * threads * 16 : 0) +
-           size_t(max_slots) * tile::dev::wpart_stride(uint32_t(nwarps), wlanes) * 8 + nwarps * 8;
+           size_t(max_slots) * tile::dev::wpart_stride(uint32_t(nwarps), wl) * 8 + nwarps * 8;
 }
 
 // ------------------------------------------------------------------ device
@@ -184,7 +184,7 @@ __device__ __forceinline__ double block_sum(double v, double* red, uint32_t nwar
     return t;
 }
 
-template <int RB>
+template <int RB, uint32_t WL>
 __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint32_t tile, double2* xbuf, double2* gval,
                                          double2* acc, double* wpart, double* red, uint32_t nwarps)
 {
@@ -208,7 +208,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         gval[g] = v;
     }
     if (rev)
-        for (uint32_t i = tid; i < nslots * wpart_stride(nwarps, A.wlanes); i += blockDim.x) wpart[i] = 0.0;
+        for (uint32_t i = tid; i < nslots * wpart_stride(nwarps, WL); i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const bool active = tid < (1u << (k - RB));
@@ -244,8 +244,8 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
     if (RB < 4)
         for (int r = 0; r < RB; ++r) own_acc[r] = make_double2(1.0, 0.0);
     const OpsEnv E{A.ops + P.op0, P.nops, A.layouts + P.lay0, A.mats + 8 * size_t(P.mat0), obase,
-                   xbuf, gval, wpart, nwarps, A.wlanes, RB == 4 ? acc + tid : own_acc, RB == 4 ? blockDim.x : 1u};
-    lay = run_ops<RB, 2>(E, lay, a, rev ? 2 : 1, active);
+                   xbuf, gval, wpart, nwarps, RB == 4 ? acc + tid : own_acc, RB == 4 ? blockDim.x : 1u};
+    lay = run_ops<RB, 2, WL>(E, lay, a, rev ? 2 : 1, active);
 
     if (!(flags & F_NOSTORE) && active) {
 #pragma unroll
@@ -266,7 +266,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
         __syncthreads();
         double* out = A.part + P.part0 + uint64_t(tile) * nslots;
         for (uint32_t s = tid; s < nslots; s += blockDim.x)
-            out[s] = slot_sum(wpart + s * wpart_stride(nwarps, A.wlanes), nwarps, A.wlanes);
+            out[s] = slot_sum<WL>(wpart + s * wpart_stride(nwarps, WL), nwarps);
     }
 }
 
@@ -274,7 +274,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& A, uint32_t pid, uint3
 // 8 amplitudes per thread and state (two CTAs of 256 threads per SM) and 168 for
 // 16 (three CTAs of 128); WIDE = 1 lets it use up to 255 (CTAs of at most 256
 // threads).  The autotuner picks by measurement.
-template <int RB, int WIDE>
+template <int RB, int WIDE, uint32_t WL>
 __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB == 4 && !WIDE ? 3 : 1)
     k_batch(const __grid_constant__ BatchArgs A)
 {
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB =
     double2* gval = smem + (size_t(1) << A.kmax);
     double2* acc = gval + A.max_groups;
     double* wpart = reinterpret_cast<double*>(acc + (RB == 4 ? RB * blockDim.x : 0));
-    double* red = wpart + size_t(A.max_slots) * wpart_stride(nwarps, A.wlanes);
+    double* red = wpart + size_t(A.max_slots) * wpart_stride(nwarps, WL);
     if (RB == 4)
         for (int r = 0; r < RB; ++r) acc[r * blockDim.x + tid] = make_double2(1.0, 0.0);
     __shared__ uint32_t s_cur, s_next;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : RB == 4 ? 128 : kMaxThreads, RB =
         if (!s_ok) break;
         for (uint32_t p = 0; p < item.npass; ++p)
             for (uint32_t t = 0; t < item.ntile; ++t)
-                run_tile<RB>(A, item.pass + p, item.tile + t, xbuf, gval, acc, wpart, red, nwarps);
+                run_tile<RB, WL>(A, item.pass + p, item.tile + t, xbuf, gval, acc, wpart, red, nwarps);
         // publish: every thread's stores are visible GPU-wide before the counter moves
         __threadfence();
         __syncthreads();
@@ -391,6 +391,7 @@ struct Config {
 struct Shape {
     uint32_t threads, rb;
     const void* kernel;
+    const void* few;             // the same with one gradient partial per warp and slot, null where kernel has one
 };
 
 Shape shape_of(const Config& c)
@@ -398,10 +399,11 @@ Shape shape_of(const Config& c)
     auto fn = [](void (*k)(BatchArgs)) { return reinterpret_cast<const void*>(k); };
     if (c.rb == 3 && c.threads >= 64) {
         const uint32_t t = c.threads / 2;
-        return Shape{t, 4, c.wide || t > 128 ? fn(k_batch<4, 1>) : fn(k_batch<4, 0>)};
+        if (c.wide || t > 128) return Shape{t, 4, fn(k_batch<4, 1, 8>), fn(k_batch<4, 1, 1>)};
+        return Shape{t, 4, fn(k_batch<4, 0, 8>), fn(k_batch<4, 0, 1>)};
     }
-    if (c.rb == 3) return Shape{c.threads, 3, fn(k_batch<3, 0>)};
-    return Shape{c.threads, 2, c.wide ? fn(k_batch<2, 1>) : fn(k_batch<2, 0>)};
+    if (c.rb == 3) return Shape{c.threads, 3, fn(k_batch<3, 0, 1>), nullptr};
+    return Shape{c.threads, 2, c.wide ? fn(k_batch<2, 1, 1>) : fn(k_batch<2, 0, 1>), nullptr};
 }
 
 struct CircuitHost {
@@ -484,6 +486,7 @@ struct qse_batch {
     qse::HostBuf host;
     // device pointers into prog / work
     BatchArgs args{};
+    const void* kernel = nullptr;
     const BPatch* patches = nullptr;
     uint32_t npatches = 0;
     const FinPass* fins = nullptr;
@@ -702,16 +705,15 @@ void build(qse_batch* b)
     }
 
     // shared memory and grid
-    // as many gradient partials per warp as leave room for three CTAs per SM; with one
-    // a pass of thousands of slots still fits (eight would stop at some 690 of them)
-    auto smem_with = [&](uint32_t wl) { return smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, wl); };
-    uint32_t wlanes = 8;
-    while (wlanes > 1 && smem_with(wlanes) > 72 * 1024) wlanes /= 2;
-    const size_t smem = smem_with(wlanes);
+    // eight gradient partials per warp where three CTAs then still fit on an SM, else
+    // one (eight would stop at some 690 slots of a pass, one holds thousands)
+    const bool few = shape.few && smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, 8) > 72 * 1024;
+    b->kernel = few ? shape.few : shape.kernel;
+    const size_t smem = smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, shape.few && !few ? 8 : 1);
     if (smem + 64 > ctx->smem_optin)
         fail(QSE_ERR_SIZE, "batch: a pass needs " + std::to_string(smem) +
                                " B of shared memory; lower max_gates or the tile size");
-    const void* kfn = shape.kernel;
+    const void* kfn = b->kernel;
     {
         cudaFuncAttributes fa{};
         QSE_CUDA(cudaFuncGetAttributes(&fa, kfn));
@@ -827,7 +829,6 @@ void build(qse_batch* b)
     A.kmax = kmax;
     A.max_groups = max_groups;
     A.max_slots = max_slots;
-    A.wlanes = wlanes;
     A.spin_limit = b->wait_limit ? b->wait_limit : kDefaultWaitPolls;
     b->d_ops = reinterpret_cast<plan::KOp*>(pd + o_ops);
     b->d_terms = reinterpret_cast<BTerm*>(pd + o_terms);
@@ -873,7 +874,7 @@ void enqueue(qse_batch* b)
     if (b->args.nitems) {
         const Shape sh = shape_of(b->cfg);
         void* args[] = {&b->args};
-        QSE_CUDA(cudaLaunchKernel(sh.kernel, dim3(b->grid), dim3(sh.threads), args, b->smem, s));
+        QSE_CUDA(cudaLaunchKernel(b->kernel, dim3(b->grid), dim3(sh.threads), args, b->smem, s));
     }
     if (b->nfins) {
         k_fin_slots<<<b->nfins, 128, 0, s>>>(b->fins, b->args.part, b->slot_occ, b->occ);

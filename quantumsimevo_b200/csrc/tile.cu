@@ -27,7 +27,7 @@ namespace {
 
 using namespace dev;
 
-template <int RB, int NS>
+template <int RB, int NS, uint32_t WL>
 __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
 {
     constexpr int R = 1 << RB;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
     const uint64_t obase = tile_base(blockIdx.x, A.outer_mask);
     group_values(A.groups, A.ngroups, A.terms, obase, gval);
     if (NS == 2)
-        for (uint32_t i = tid; i < A.nslots * wpart_stride(nwarps, A.wlanes); i += blockDim.x) wpart[i] = 0.0;
+        for (uint32_t i = tid; i < A.nslots * wpart_stride(nwarps, WL); i += blockDim.x) wpart[i] = 0.0;
     __syncthreads();
 
     const plan::LayoutRec* lay = A.layouts + A.layout0;
@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
         if (NS == 2) a[NS - 1][j] = A.lam[idx];
     }
 
-    OpsEnv E{A.ops, A.nops, A.layouts, A.mats, obase, xbuf, gval, wpart, nwarps, A.wlanes, acc + tid, blockDim.x};
-    lay = run_ops<RB, NS>(E, lay, a, NS, true);
+    OpsEnv E{A.ops, A.nops, A.layouts, A.mats, obase, xbuf, gval, wpart, nwarps, acc + tid, blockDim.x};
+    lay = run_ops<RB, NS, WL>(E, lay, a, NS, true);
 
     for (int i = 0; i < RB; ++i) rg[i] = uint64_t(1) << lay->preg[i];
     base = thread_base<uint64_t>(lay, obase, tid);
@@ -74,26 +74,26 @@ __global__ void __launch_bounds__(256, 2) k_tile(const PassArgs A)
         __syncthreads();
         for (uint32_t s = tid; s < A.nslots; s += blockDim.x)
             A.slot_partial[uint64_t(s) * gridDim.x + blockIdx.x] =
-                slot_sum(wpart + s * wpart_stride(nwarps, A.wlanes), nwarps, A.wlanes);
+                slot_sum<WL>(wpart + s * wpart_stride(nwarps, WL), nwarps);
     }
 }
 
-template <int RB, int NS>
+template <int RB, int NS, uint32_t WL>
 void launch_t(qse_ctx* ctx, const PassArgs& a, uint32_t n, size_t smem)
 {
     static bool configured[64] = {false};
     int dev = ctx->device;
     if (!configured[dev & 63]) {
         cudaFuncAttributes fa{};
-        QSE_CUDA(cudaFuncGetAttributes(&fa, k_tile<RB, NS>));
-        QSE_CUDA(cudaFuncSetAttribute(k_tile<RB, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        QSE_CUDA(cudaFuncGetAttributes(&fa, k_tile<RB, NS, WL>));
+        QSE_CUDA(cudaFuncSetAttribute(k_tile<RB, NS, WL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(ctx->smem_optin - fa.sharedSizeBytes)));
         configured[dev & 63] = true;
     }
     uint32_t threads = 1u << (a.k - RB);
     uint64_t grid = uint64_t(1) << (n - a.k);
     cudaEvent_t ev_stop = pass_timer_begin(ctx);
-    k_tile<RB, NS><<<unsigned(grid), threads, smem, ctx->stream>>>(a);
+    k_tile<RB, NS, WL><<<unsigned(grid), threads, smem, ctx->stream>>>(a);
     QSE_CUDA(cudaGetLastError());
     pass_timer_end(ctx, ev_stop);
     count_launch(ctx);
@@ -122,27 +122,26 @@ void pass_timer_end(qse_ctx* ctx, cudaEvent_t stop)
     if (stop) QSE_CUDA(cudaEventRecord(stop, ctx->stream));
 }
 
-size_t pass_smem_bytes(uint32_t k, uint32_t ngroups, uint32_t nslots, uint32_t rb, int nstates, uint32_t wlanes)
+size_t pass_smem_bytes(uint32_t k, uint32_t ngroups, uint32_t nslots, uint32_t rb, int nstates, uint32_t wl)
 {
     size_t threads = size_t(1) << (k - rb);
     size_t b = (size_t(1) << k) * 16 + size_t(ngroups) * 16 + size_t(rb) * threads * 16;
-    if (nstates == 2) b += size_t(nslots) * dev::wpart_stride(uint32_t((threads + 31) / 32), wlanes) * 8;
+    if (nstates == 2) b += size_t(nslots) * dev::wpart_stride(uint32_t((threads + 31) / 32), wl) * 8;
     return b;
 }
 
-void launch_pass(qse_ctx* ctx, const PassArgs& args, uint32_t n, uint32_t rb, int nstates)
+void launch_pass(qse_ctx* ctx, const PassArgs& a, uint32_t n, uint32_t rb, int nstates)
 {
-    // as many gradient partials per warp as leave room for two CTAs per SM (eight per
-    // warp would not fit at all beyond some 350 slots)
-    PassArgs a = args;
-    a.wlanes = 8;
-    while (a.wlanes > 1 && pass_smem_bytes(a.k, a.ngroups, a.nslots, rb, nstates, a.wlanes) > 100 * 1024) a.wlanes /= 2;
-    size_t smem = pass_smem_bytes(a.k, a.ngroups, a.nslots, rb, nstates, a.wlanes);
+    // eight gradient partials per warp where two CTAs then still fit on an SM, else one
+    // (eight would not fit at all beyond some 350 slots)
+    const bool few = nstates == 2 && pass_smem_bytes(a.k, a.ngroups, a.nslots, rb, nstates, 8) > 100 * 1024;
+    size_t smem = pass_smem_bytes(a.k, a.ngroups, a.nslots, rb, nstates, few ? 1 : 8);
     if (smem > ctx->smem_optin) fail(QSE_ERR_SIZE, "tile pass needs more shared memory than the device offers");
     if (n - a.k > 31) fail(QSE_ERR_SIZE, "too many tiles for one launch");
-    if (rb == 4 && nstates == 1) launch_t<4, 1>(ctx, a, n, smem);
-    else if (rb == 3 && nstates == 2) launch_t<3, 2>(ctx, a, n, smem);
-    else if (rb == 3 && nstates == 1) launch_t<3, 1>(ctx, a, n, smem);
+    if (rb == 4 && nstates == 1) launch_t<4, 1, 8>(ctx, a, n, smem);
+    else if (rb == 3 && nstates == 2 && few) launch_t<3, 2, 1>(ctx, a, n, smem);
+    else if (rb == 3 && nstates == 2) launch_t<3, 2, 8>(ctx, a, n, smem);
+    else if (rb == 3 && nstates == 1) launch_t<3, 1, 8>(ctx, a, n, smem);
     else fail(QSE_ERR_INVALID, "unsupported tile configuration");
 }
 

@@ -289,39 +289,40 @@ struct OpsEnv {
     uint64_t obase;
     double2* xbuf;                    // 2^k slots
     const double2* gval;              // group values of this CTA: unit phases
-    double* wpart;                    // gradient partials (NS == 2), wpart_stride(nwarps, wlanes) per slot
-    uint32_t nwarps, wlanes;
+    double* wpart;                    // gradient partials (NS == 2), wpart_stride(nwarps, WL) per slot
+    uint32_t nwarps;
     double2* acc;                     // phase accumulators of register bit p at acc[p * acc_stride] (1 on entry and exit)
     uint32_t acc_stride;
 };
 
-// Gradient partials of a slot: wlanes (8, 4, 2 or 1) per warp (add_partial), and,
-// above one, a double of padding so that the threads that sum a slot each
-// (slot_sum) hit distinct banks.  The launch takes as many as fit in shared memory.
-__host__ __device__ constexpr uint32_t wpart_stride(uint32_t nwarps, uint32_t wlanes)
+// Gradient partials of a slot: WL (8 or 1) per warp (add_partial), and, with 8, a
+// double of padding so that the threads that sum a slot each (slot_sum) hit distinct
+// banks.  The launch takes 8 where they leave room for its CTAs in shared memory, else
+// 1; a compile-time choice, since a runtime one costs the batched kernel 2 %.
+__host__ __device__ constexpr uint32_t wpart_stride(uint32_t nwarps, uint32_t wl)
 {
-    return wlanes * nwarps + (wlanes > 1 ? 1 : 0);
+    return wl * nwarps + (wl > 1 ? 1 : 0);
 }
 
-// Adds a gate's per-thread sums to its slot: with wlanes 8, two exchange steps
-// leave eight sums a warp, and the rest waits for the end of the tile, where all
-// slots are summed at once (five dependent steps per gate were a tenth of a
-// reverse tile's latency).
-__device__ __forceinline__ void add_partial(double v, double* slot, uint32_t wlanes)
+// Adds a gate's per-thread sums to its slot: with WL 8, two exchange steps leave
+// eight sums a warp, and the rest waits for the end of the tile, where all slots are
+// summed at once (five dependent steps per gate were a tenth of a reverse tile's
+// latency).
+template <uint32_t WL>
+__device__ __forceinline__ void add_partial(double v, double* slot)
 {
     const uint32_t nb = blockDim.x, tid = threadIdx.x, lane = tid & 31;
     const unsigned mask = nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u);
 #pragma unroll
-    for (uint32_t o = 16; o >= 8; o >>= 1)
+    for (uint32_t o = 16; o >= WL; o >>= 1)
         if (o < nb) v += __shfl_xor_sync(mask, v, o);
-    for (uint32_t o = 4; o >= wlanes; o >>= 1)   // only where the launch had to take fewer
-        if (o < nb) v += __shfl_xor_sync(mask, v, o);
-    if (lane < wlanes) slot[(tid >> 5) * wlanes + lane] += v;
+    if (lane < WL) slot[(tid >> 5) * WL + lane] += v;
 }
-__device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps, uint32_t wlanes)
+template <uint32_t WL>
+__device__ __forceinline__ double slot_sum(const double* slot, uint32_t nwarps)
 {
     double v = 0.0;
-    for (uint32_t i = 0; i < wlanes * nwarps; ++i) v += slot[i];
+    for (uint32_t i = 0; i < WL * nwarps; ++i) v += slot[i];
     return v;
 }
 
@@ -354,7 +355,7 @@ static_assert(offsetof(KOp, kind) == 0 && offsetof(KOp, p) == 1 && offsetof(KOp,
 // Threads with active == false hold zeros, never touch the exchange buffer
 // and add nothing to the gradient partials; they only join the barriers
 // (a CTA wider than the tile of a small state).
-template <int RB, int NS>
+template <int RB, int NS, uint32_t WL>
 __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const plan::LayoutRec* lay,
                                                          double2 (&a)[NS][1 << RB], int nact, bool active)
 {
@@ -523,7 +524,7 @@ __device__ __forceinline__ const plan::LayoutRec* run_ops(const OpsEnv& E, const
                             if ((j & op.f()) == op.f()) part += im_ls(a[1][j], a[0][j]);
                     }
                 }
-                add_partial(part * op.a(), E.wpart + op.g() * wpart_stride(E.nwarps, E.wlanes), E.wlanes);
+                add_partial<WL>(part * op.a(), E.wpart + op.g() * wpart_stride(E.nwarps, WL));
             }
             break;
         }

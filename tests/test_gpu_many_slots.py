@@ -1,7 +1,7 @@
-"""Reverse passes with many gradient slots: the interpreter keeps 8, 4, 2 or 1
-partial sums per warp and slot, as many as fit in shared memory.  Values and
+"""Reverse passes with many gradient slots: the interpreter keeps 8 or 1
+partial sums per warp and slot, 8 where they fit in shared memory.  Values and
 gradients against the FP64 oracle's adjoint (1e-10, as the other gradient
-tests), at slot counts on both sides of each change, up to counts that only fit
+tests), at slot counts on both sides of the change, up to counts that only fit
 with one partial per warp."""
 import numpy as np
 import pytest
@@ -37,7 +37,7 @@ def expected(n, ops, params, obs):
     return O.adjoint(n, ops, params, o)
 
 
-# default shape (128 threads): 8 partials up to some 120 slots of 6 qubits, 1 beyond 500
+# default shape (128 threads): 8 partials at 60 slots, 1 beyond some 200
 @pytest.mark.parametrize("cfg", [None, BatchConfig(threads=32, reg_bits=2), BatchConfig(threads=512, reg_bits=3)])
 @pytest.mark.parametrize("gates", [60, 300, 700, 1500])
 def test_batched_circuits(cfg, gates):
