@@ -324,16 +324,18 @@ QSE_API int qse_batch_autotune(qse_batch* b, const char* cache_path);
 QSE_API int qse_batch_use_graph(qse_batch* b, int enabled);
 
 typedef struct qse_batch_config {
-    uint32_t threads;       /* CTA size, a power of two in 32..512                       */
-    uint32_t reg_bits;      /* 2^reg_bits amplitudes per thread: 2 or 3                   */
-                            /* tile qubits k = log2(threads) + reg_bits                   */
+    uint32_t threads;       /* a power of two in 32..512                                  */
+    uint32_t reg_bits;      /* 2 or 3; tile qubits k = log2(threads) + reg_bits.  CTAs    */
+                            /* have `threads` threads with 2^reg_bits amplitudes each, or */
+                            /* (reg_bits 3, threads >= 64) half of them with 16 each      */
     uint32_t max_gates;     /* non-diagonal gates per pass, 0 = no cap                    */
     uint32_t chain_tiles;   /* circuits with at most this many tiles per pass run as one
-                               work item (one CTA, start to end); >= 1                    */
+                               work item (one CTA, start to end), unless one alone would
+                               hold up the batch; >= 1                                    */
     uint32_t ctas_per_sm;   /* persistent CTAs per SM, 0 = as many as fit                 */
     uint32_t grad_slots;    /* gradient slots per pass, 0 = no cap                        */
-    uint32_t wide_regs;     /* 1: up to 255 registers per thread (threads <= 256, one CTA
-                               per SM); 0: 128 registers (two CTAs of 256 per SM)         */
+    uint32_t wide_regs;     /* 1: up to 255 registers per thread (threads <= 256); 0: 128,
+                               or 168 with 16 amplitudes per thread                       */
 } qse_batch_config;
 QSE_API int qse_batch_set_config(qse_batch* b, const qse_batch_config* cfg);
 /* Bound of the persistent kernel's dependency waits: a work item polls the

@@ -22,8 +22,8 @@ from .circuit import Device
 
 @dataclass
 class BatchConfig:
-    threads: int = 256      # CTA size (power of two, 32..512)
-    reg_bits: int = 3       # 2^reg_bits amplitudes per thread; tile qubits = log2(threads) + reg_bits
+    threads: int = 256      # power of two, 32..512; with reg_bits 3 the CTAs have half as many (16 amplitudes each)
+    reg_bits: int = 3       # 2 or 3; tile qubits = log2(threads) + reg_bits
     max_gates: int = 0      # non-diagonal gates per pass, 0 = no cap
     chain_tiles: int = 1    # circuits with <= this many tiles run start to end in one CTA
     ctas_per_sm: int = 0    # 0 = as many as fit
