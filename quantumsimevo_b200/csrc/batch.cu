@@ -487,6 +487,7 @@ struct qse_batch {
     // device pointers into prog / work
     BatchArgs args{};
     const void* kernel = nullptr;
+    uint32_t threads = 0;         // CTA size of the built batch
     const BPatch* patches = nullptr;
     uint32_t npatches = 0;
     const FinPass* fins = nullptr;
@@ -705,11 +706,15 @@ void build(qse_batch* b)
     }
 
     // shared memory and grid
+    // No more threads than the widest tile uses: on circuits narrower than the tiles
+    // the rest of a CTA only waits at barriers, and its registers keep other CTAs off
+    // the SM (512 circuits of 6 to 10 qubits: 128 threads 732 us, 64 threads 540).
+    b->threads = std::min(shape.threads, std::max(32u, 1u << (kmax - std::min(kmax, shape.rb))));
     // eight gradient partials per warp where three CTAs then still fit on an SM, else
     // one (eight would stop at some 690 slots of a pass, one holds thousands)
-    const bool few = shape.few && smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, 8) > 72 * 1024;
+    const bool few = shape.few && smem_bytes(kmax, max_groups, max_slots, b->threads, shape.rb, 8) > 72 * 1024;
     b->kernel = few ? shape.few : shape.kernel;
-    const size_t smem = smem_bytes(kmax, max_groups, max_slots, shape.threads, shape.rb, shape.few && !few ? 8 : 1);
+    const size_t smem = smem_bytes(kmax, max_groups, max_slots, b->threads, shape.rb, shape.few && !few ? 8 : 1);
     if (smem + 64 > ctx->smem_optin)
         fail(QSE_ERR_SIZE, "batch: a pass needs " + std::to_string(smem) +
                                " B of shared memory; lower max_gates or the tile size");
@@ -721,7 +726,7 @@ void build(qse_batch* b)
                                       int(ctx->smem_optin - fa.sharedSizeBytes)));
     }
     int occ_blocks = 0;
-    QSE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blocks, kfn, int(shape.threads), smem));
+    QSE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blocks, kfn, int(b->threads), smem));
     if (occ_blocks < 1) fail(QSE_ERR_SIZE, "batch: kernel configuration does not fit on an SM");
     uint32_t per_sm = uint32_t(occ_blocks);
     if (cf.ctas_per_sm) per_sm = std::min(per_sm, cf.ctas_per_sm);
@@ -872,9 +877,8 @@ void enqueue(qse_batch* b)
         QSE_CUDA(cudaGetLastError());
     }
     if (b->args.nitems) {
-        const Shape sh = shape_of(b->cfg);
         void* args[] = {&b->args};
-        QSE_CUDA(cudaLaunchKernel(b->kernel, dim3(b->grid), dim3(sh.threads), args, b->smem, s));
+        QSE_CUDA(cudaLaunchKernel(b->kernel, dim3(b->grid), dim3(b->threads), args, b->smem, s));
     }
     if (b->nfins) {
         k_fin_slots<<<b->nfins, 128, 0, s>>>(b->fins, b->args.part, b->slot_occ, b->occ);

@@ -1,4 +1,5 @@
-"""Reverse passes with many gradient slots: the interpreter keeps 8 or 1
+"""Batched circuits at the limits of a CTA (as many threads as the widest tile
+uses), and reverse passes with many gradient slots: the interpreter keeps 8 or 1
 partial sums per warp and slot, 8 where they fit in shared memory.  Values and
 gradients against the FP64 oracle's adjoint (1e-10, as the other gradient
 tests), at slot counts on both sides of the change, up to counts that only fit
@@ -50,6 +51,27 @@ def test_batched_circuits(cfg, gates):
     vw, gw = expected(n, ops, params, obs)
     assert abs(v[0] - vw) <= TOL
     assert np.max(np.abs(g - gw)) <= TOL
+
+
+# CTAs have no more threads than the widest tile: from the narrowest circuits, over
+# each CTA size, up to the configured one
+@pytest.mark.parametrize("cfg", [None, BatchConfig(threads=512, reg_bits=3), BatchConfig(threads=256, reg_bits=2)])
+@pytest.mark.parametrize("widths", [(4,), (5, 6), (4, 8, 9), (6, 10), (11, 4), (12, 4)])
+def test_batches_of_narrow_circuits(cfg, widths):
+    circs, params, vw, gw = [], [], [], []
+    for i, n in enumerate(widths):
+        ops, p, obs = circuit(n, 12 * n, 7 * i + n, phases=False)
+        circs.append((n, ops, len(p), obs))
+        params.append(p)
+        v, g = expected(n, ops, p, obs)
+        vw.append(v)
+        gw.append(g)
+    b = Batch(circs, Device(0))
+    if cfg is not None:
+        b.config = cfg
+    v, g = b.run(np.concatenate(params))
+    assert np.max(np.abs(v - np.array(vw))) <= TOL
+    assert np.max(np.abs(g - np.concatenate(gw))) <= TOL
 
 
 @pytest.mark.parametrize("n,gates", [(5, 90), (10, 300), (11, 500), (12, 1000)])
