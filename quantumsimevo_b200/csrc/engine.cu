@@ -1065,6 +1065,7 @@ constexpr int kRB = 256;
 constexpr uint32_t kObsBits = 4;
 constexpr uint32_t kObsLow = 8;      // kRB = 2^kObsLow threads hold the bits below
 constexpr int kObsR = 1 << kObsBits;
+constexpr size_t kObsMaxTerms = 4096;   // 64 KiB of shared memory: two CTAs still fit on an SM
 struct ObsFirst {
     uint16_t first[kObsR + 1];
 };
@@ -1197,7 +1198,7 @@ ObsDev upload_obs(qse_state* st, const qse_observable* obs, char* dbase, char* h
     uint32_t at[kObsR];
     for (int p = 0; p < kObsR; ++p) {
         at[p] = o.f.first[p];
-        o.f.first[p + 1] = uint16_t(o.f.first[p] + count[p]);   // at most 4096 terms
+        o.f.first[p + 1] = uint16_t(o.f.first[p] + count[p]);   // at most kObsMaxTerms
     }
     for (size_t t = 0; t < obs->nterms; ++t) {
         const uint32_t k = at[pattern(phys[t])]++;
@@ -1228,7 +1229,7 @@ ObsRun launch_obs(qse_state* st, const qse_observable* obs, double2* lam)
 {
     materialize(st);
     qse_ctx* ctx = st->ctx;
-    if (obs->nterms > 4096) fail(QSE_ERR_SIZE, "observable has too many terms");
+    if (obs->nterms > kObsMaxTerms) fail(QSE_ERR_SIZE, "observable has too many terms");
     const uint64_t size = st->size();
     const uint64_t chunks = (size + uint64_t(kRB) * kObsR - 1) / (uint64_t(kRB) * kObsR);
     const unsigned grid = unsigned(std::min<uint64_t>(chunks, uint64_t(ctx->num_sms) * 8));
@@ -1241,7 +1242,10 @@ ObsRun launch_obs(qse_state* st, const qse_observable* obs, double2* lam)
     ObsDev o = upload_obs(st, obs, d, h);
     QSE_CUDA(cudaEventRecord(ctx->small_event, ctx->stream));
     double* partial = reinterpret_cast<double*>(d + obytes);
-    k_obs<<<grid, kRB, 16 * obs->nterms, ctx->stream>>>(reinterpret_cast<const double2*>(st->amp), lam, size, o.z, o.w,
+    const size_t smem = 16 * obs->nterms;
+    if (smem > 47 * 1024)   // beyond what a launch gets unasked: 48 KiB, some of it the kernel's static arrays
+        QSE_CUDA(cudaFuncSetAttribute(k_obs, cudaFuncAttributeMaxDynamicSharedMemorySize, int(16 * kObsMaxTerms)));
+    k_obs<<<grid, kRB, smem, ctx->stream>>>(reinterpret_cast<const double2*>(st->amp), lam, size, o.z, o.w,
                                                         o.nt, o.f, o.c, partial);
     QSE_CUDA(cudaGetLastError());
     count_launch(ctx);

@@ -30,3 +30,59 @@ def test_expectation_matches_plain_sum(n, nterms):
     want = float(np.sum(o * (psi.real ** 2 + psi.imag ** 2)))
     # |O| <= 0.25 + sum |w|: a few hundred roundings of 2^-53 of that, with the norm 1
     assert abs(c.expectation(z, w, 0.25) - want) <= 1e-13 * (0.25 + float(np.abs(w).sum()))
+
+
+def _plain(psi, z, w, c):
+    """sum_x (c + sum_t w_t (-1)^popcount(x & z_t)) |psi_x|^2 in doubles."""
+    i = np.arange(psi.size, dtype=np.uint64)
+    o = np.full(psi.size, c)
+    for m, x in zip(z, w):
+        o += np.where(np.bitwise_count(i & m) & 1, -x, x)
+    return float(np.sum(o * (psi.real ** 2 + psi.imag ** 2)))
+
+
+# the terms sit in shared memory, 16 B each: a launch gets 48 KiB unasked, some of it
+# taken by the kernel's static arrays
+@pytest.mark.parametrize("nterms", [3007, 3008, 3009, 3068, 3069, 3072, 3073, 4096])
+def test_as_many_terms_as_are_accepted(nterms):
+    from quantumsimevo_b200.circuit import Circuit
+
+    n = 13
+    rng = np.random.default_rng(nterms)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    psi /= np.linalg.norm(psi)
+    c = Circuit(n)
+    c.state.upload(psi)
+    z = rng.integers(0, 1 << n, nterms, dtype=np.uint64)
+    w = rng.standard_normal(nterms)
+    # up to 4096 terms added one by one: as many roundings of 2^-53 of sum |w|, with the norm 1
+    assert abs(c.expectation(z, w, 0.25) - _plain(psi, z, w, 0.25)) <= 1e-12 * (0.25 + float(np.abs(w).sum()))
+
+
+def test_too_many_terms_is_a_size_error():
+    from quantumsimevo_b200 import _lib as L
+    from quantumsimevo_b200.circuit import Circuit
+
+    c = Circuit(5)
+    with pytest.raises(L.QseError) as e:
+        c.expectation(np.ones(4097, dtype=np.uint64), np.ones(4097), 0.0)
+    assert e.value.status == 5   # QSE_ERR_SIZE
+    assert abs(c.expectation([1], [1.0], 0.0) - 1.0) <= 1e-15
+
+
+def test_gradient_with_as_many_terms_as_are_accepted():
+    import oracle_ffi as O
+    from quantumsimevo_b200 import _lib as L
+    from quantumsimevo_b200 import workloads as W
+    from quantumsimevo_b200.autograd import ParametrizedCircuit
+
+    n = 10
+    ops, params, _, _ = W.qaoa_maxcut(n, 2, seed=5)
+    rng = np.random.default_rng(6)
+    z = [int(x) for x in rng.integers(1, 1 << n, 4096)]
+    w = [float(x) / 64.0 for x in rng.standard_normal(4096)]
+    v, g = ParametrizedCircuit(n, ops, z, w, 0.5).value_and_grad(params)
+    obs, keep = L.observable(z, w, 0.5)
+    vw, gw = O.adjoint(n, ops, params, obs)
+    assert abs(v - vw) <= 1e-10
+    assert np.max(np.abs(g - gw)) <= 1e-10
