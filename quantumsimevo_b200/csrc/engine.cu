@@ -361,11 +361,12 @@ uint32_t tile_qubits_for(const qse_ctx* ctx, uint32_t n, uint32_t rb, uint32_t k
 // more per distinct kernel) when a pass is expensive, i.e. on large states, or
 // when few of a plan's kernels are new.  A deep circuit on a small state can
 // need hundreds of distinct kernels; its plan runs on the interpreter instead.
+// A small state's plan in smaller tiles has more kernels for the same gates, each
+// compiled faster (a quarter of the amplitudes per thread: 16-qubit layered
+// rotations 0.9 s for all 18 kernels, 4.8 s for 8 in 12-qubit tiles), so what the
+// compilation may cost is counted in the kernels of 12-qubit tiles.
 constexpr uint32_t kJitAlwaysQubits = 22;
 constexpr size_t kJitMaxNewKernels = 32;
-// ... kernels with 8 amplitudes per thread (small states) compile about five times
-// faster (16-qubit layered rotations: 0.9 s for all passes instead of 4.8)
-constexpr size_t kJitMaxNewSmall = 96;
 // States of at most kSmallQubits qubits hold 8 amplitudes per thread in tiles of
 // 2^11 (up to kTile11Qubits, where more passes cost more than fuller SMs give)
 // or 2^10: with 32 per thread and 2^12 they are a few CTAs of four warps each
@@ -432,28 +433,40 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     e->numbers = std::move(numbers);
     e->opt = opt;
     e->pl = plan::build(gates, st->n, st->perm, opt);
-    const plan::Plan& pl = e->pl;
     if (e->use_jit) {
-        e->srcs.reserve(pl.passes.size());
-        // the last pass may also write the probabilities in logical order
-        uint8_t lpos[64] = {0};
-        for (uint32_t q = 0; q < st->n; ++q) lpos[pl.perm_final[q]] = uint8_t(q);
-        for (size_t i = 0; i < pl.passes.size(); ++i) {
-            const bool basis_in = i == 0 && ns == 1 && st->lazy_basis;
-            const bool prob = prob_out && ns == 1 && i + 1 == pl.passes.size();
-            e->srcs.push_back(jit::generate(pl.passes[i], ns, basis_in, ctx->jit == 2, st->n >= jit::kPreGroupQubits,
+        auto sources = [&](const plan::Plan& p, std::vector<jit::Source>& out) {
+            // the last pass may also write the probabilities in logical order
+            uint8_t lpos[64] = {0};
+            for (uint32_t q = 0; q < st->n; ++q) lpos[p.perm_final[q]] = uint8_t(q);
+            out.reserve(p.passes.size());
+            for (size_t i = 0; i < p.passes.size(); ++i) {
+                const bool basis_in = i == 0 && ns == 1 && st->lazy_basis;
+                const bool prob = prob_out && ns == 1 && i + 1 == p.passes.size();
+                out.push_back(jit::generate(p.passes[i], ns, basis_in, ctx->jit == 2, st->n >= jit::kPreGroupQubits,
                                             basis_in ? st->lazy_umask : 0, prob ? lpos : nullptr,
                                             basis_in ? st->lazy_pmask : 0));
-        }
-        if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > (opt.rb <= 3 ? kJitMaxNewSmall : kJitMaxNewKernels)) {
-            e->use_jit = false;
-            e->srcs.clear();
-            opt.unit_rot = false;
-            opt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
-            opt.rb_first = 0;
-            if (ns == 1) opt.k = tile_qubits_for(ctx, st->n, 4, 12);
-            e->opt = opt;
-            e->pl = plan::build(gates, st->n, st->perm, opt);
+            }
+        };
+        sources(e->pl, e->srcs);
+        if (st->n < kJitAlwaysQubits && jit::count_uncached(e->srcs) > kJitMaxNewKernels) {
+            // the same gates as the interpreter would run them
+            plan::Options iopt = opt;
+            iopt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
+            iopt.rb_first = 0;
+            if (ns == 1) iopt.k = tile_qubits_for(ctx, st->n, 4, 12);
+            bool interpret = iopt.k == opt.k;
+            if (!interpret) {
+                std::vector<jit::Source> full;
+                sources(plan::build(gates, st->n, st->perm, iopt), full);
+                interpret = jit::count_uncached(full) > kJitMaxNewKernels;
+            }
+            if (interpret) {
+                iopt.unit_rot = false;
+                e->use_jit = false;
+                e->srcs.clear();
+                e->opt = iopt;
+                e->pl = plan::build(gates, st->n, st->perm, iopt);
+            }
         }
     }
     plan_cache_insert(ctx, e);
