@@ -424,7 +424,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     if (auto hit = plan_cache_find(ctx, e->key, e->hash)) {
         if (hit->numbers.size() != numbers.size() ||
             std::memcmp(hit->numbers.data(), numbers.data(), numbers.size() * sizeof(double)) != 0) {
-            plan::bind_angles(hit->pl, gates, hit->opt);
+            plan::bind_angles(hit->pl, gates, hit->opt);   // sets all of them or throws; nothing below throws
             for (size_t i = 0; i < hit->srcs.size(); ++i) jit::bind_params(hit->srcs[i], hit->pl.passes[i]);
             hit->numbers = std::move(numbers);
         }

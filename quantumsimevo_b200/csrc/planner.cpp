@@ -605,8 +605,14 @@ private:
 void bind_gates(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
 {
     double cr = 1.0, ci = 0.0;   // the constant deferred by the passes so far
+    // the only allocation, ahead of the first number that changes: a call that runs
+    // out of memory leaves the plan as it was
+    std::vector<double> divisor;
+    size_t most = 0;
+    for (const PassProgram& P : plan.passes) most = std::max(most, P.op_angles.size());
+    divisor.reserve(most);
     for (PassProgram& P : plan.passes) {
-        std::vector<double> divisor;
+        divisor.clear();
         for (const AngleRef& r : P.op_angles) {
             const double c = std::cos(gates[r.src].theta / 2.0), s = std::sin(gates[r.src].theta / 2.0);
             const bool by_c = std::fabs(c) >= std::fabs(s);

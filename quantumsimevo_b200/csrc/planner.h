@@ -197,7 +197,8 @@ Plan build(const std::vector<Gate>& gates, uint32_t n, const uint32_t* perm_in, 
 // Everything in a plan but its numbers depends on the gates' types, qubits and
 // gradient ids only: this sets the numbers (angles, matrices, constants) of a
 // plan built for gates that differ from these in theta and m at most, to what
-// build() gives for them, bit for bit.
+// build() gives for them, bit for bit.  When memory runs out it throws with every
+// number as it was.
 void bind_angles(Plan& plan, const std::vector<Gate>& gates, const Options& opt);
 
 // Planner-only debug view used by the CPU tests: for each pass, the tile
