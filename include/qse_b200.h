@@ -136,7 +136,8 @@ QSE_API int qse_ctx_synchronize(qse_ctx* ctx);
 /* fused-planner knobs: tile qubits (10..12; 12, the default, lets states of at
  * most 20 qubits run smaller tiles), cap on non-diagonal gates per pass
  * (0 = none; with specialised pass kernels at most 256, which bounds their
- * compile time), fusion on/off (off = one kernel per gate, the plain method). */
+ * compile time), fusion: 0 = one kernel per gate (the plain method), 1 = on,
+ * 2 = on, and tile_qubits 12 means 12 on small states too. */
 QSE_API int qse_ctx_set_fusion(qse_ctx* ctx, int enabled, int tile_qubits, int max_gates_per_pass);
 /* 0 = sequential-rounding-exact CDF (default), 1 = plain parallel scan */
 QSE_API int qse_ctx_set_sample_mode(qse_ctx* ctx, int mode);

@@ -44,8 +44,12 @@ class Device:
             d = cls._default[device] = Device(device)
         return d
 
-    def set_fusion(self, enabled: bool = True, tile_qubits: int = 0, max_gates_per_pass: int = 0) -> None:
-        check(lib.qse_ctx_set_fusion(self.handle, 1 if enabled else 0, int(tile_qubits), int(max_gates_per_pass)))
+    def set_fusion(self, enabled: bool = True, tile_qubits: int = 0, max_gates_per_pass: int = 0,
+                   exact_tiles: bool = False) -> None:
+        """Fusion on or off, tile qubits (0: as they are), non-diagonal gates per pass.
+        With 12 tile qubits states of at most 20 qubits run smaller tiles, unless exact_tiles."""
+        mode = 0 if not enabled else 2 if exact_tiles else 1
+        check(lib.qse_ctx_set_fusion(self.handle, mode, int(tile_qubits), int(max_gates_per_pass)))
 
     def synchronize(self) -> None:
         check(lib.qse_ctx_synchronize(self.handle))

@@ -602,7 +602,7 @@ plan::Options fused_options(const qse_ctx* ctx, uint32_t n, bool compact_input =
     // flight, and half the code to fetch (27-qubit random layers 0.72-0.83 ms a
     // pass, with 32 per thread 1.12-1.24).
     if (ctx->jit == 1 && opt.k == 12 && compact_input) opt.rb_first = 5;
-    if (ctx->jit == 1 && ctx->tile_qubits == 12 && n <= kSmallQubits) {
+    if (ctx->jit == 1 && ctx->tile_qubits == 12 && !ctx->exact_tiles && n <= kSmallQubits) {
         opt.k = std::min(n <= kTile11Qubits ? 11u : 10u, n);
         opt.rb = 3;
     }

@@ -58,6 +58,7 @@ struct qse_ctx {
     int jit = 1;             // specialised NVRTC pass kernels (0: generic interpreter kernel,
                              // 2: specialised, with the streamed persistent kernel where it applies)
     int tile_qubits = 12;    // upper limit (small states take smaller tiles: engine.cu, fused_options)
+    bool exact_tiles = false;   // ... unless this is set
     int max_gates_per_pass = 0;
     int sample_mode = 0;
     uint64_t launches = 0;
