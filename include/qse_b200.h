@@ -239,10 +239,12 @@ QSE_API int qse_plan_describe(uint32_t nqubits, const qse_op* ops, size_t nops, 
  * while two thread groups compute). */
 QSE_API int qse_ctx_set_jit(qse_ctx* ctx, int enabled);
 /* Generates and compiles (no GPU needed, nothing loaded) every distinct pass
- * kernel the planner makes for ops: nstates 1 = forward passes, 2 = adjoint
- * reverse passes, 3 = forward passes as streamed kernels where a pass allows
- * it (qse_ctx_set_jit mode 2).  *source_bytes receives the total generated
- * source size. */
+ * kernel that an execute of ops makes on a context with default settings (or
+ * with tiles of exactly tile_qubits): nstates 1 = forward passes, on states of
+ * 24 qubits and more also the first one as it reads a compact state; 2 =
+ * adjoint reverse passes; 3 = forward passes as streamed kernels where a pass
+ * allows it (qse_ctx_set_jit mode 2).  *source_bytes receives the total
+ * generated source size. */
 QSE_API int qse_plan_compile(uint32_t nqubits, const qse_op* ops, size_t nops, const double* params,
                              size_t nparams, uint32_t tile_qubits, int nstates, size_t* source_bytes);
 

@@ -603,20 +603,30 @@ int qse_plan_compile(uint32_t nqubits, const qse_op* ops, size_t nops, const dou
     }
     uint32_t perm[64];
     for (uint32_t q = 0; q < 64; ++q) perm[q] = q;
-    qse::plan::Options opt;
-    opt.k = std::min<uint32_t>(tile_qubits ? tile_qubits : (nstates == 2 ? 11 : 12), nqubits);
-    opt.rb = nstates == 2 && opt.k != 11 ? 3 : 4;   // as the engine plans large states
-    opt.grads = nstates == 2;
-    opt.acc_mul = opt.unit_rot = true;
-    opt.max_gates = qse::plan::kJitMaxGates;
-    if (nstates == 2) opt.max_terms = 512;
-    qse::plan::Plan pl = qse::plan::build(gates, nqubits, perm, opt);
+    qse::plan::Settings set;   // a context's, with the tile size asked for
+    set.jit = streamed ? 2 : 1;
+    if (tile_qubits) {
+        set.tile_qubits = int(std::min<uint32_t>(tile_qubits, 12));
+        set.exact_tiles = true;
+    }
+    qse::plan::Options opt = nstates == 2 ? qse::plan::adjoint_options(set, nqubits)
+                                          : qse::plan::forward_options(set, nqubits, false);
+    opt.rb = std::min(opt.rb, opt.k);
     size_t total = 0;
     std::set<std::string> done;   // identical passes share one kernel, as in execution
-    for (const auto& p : pl.passes) {
-        qse::jit::Source s = qse::jit::generate(p, nstates, false, streamed, nqubits >= qse::jit::kPreGroupQubits);
+    auto compile = [&](const qse::jit::Source& s) {
         total += s.code.size();
         if (done.insert(s.code).second) qse::jit::compile_only(s);
+    };
+    const bool pre_groups = nqubits >= qse::jit::kPreGroupQubits;
+    const qse::plan::Plan pl = qse::plan::build(gates, nqubits, perm, opt);
+    for (const auto& p : pl.passes) compile(qse::jit::generate(p, nstates, false, streamed, pre_groups));
+    // large states also start from a compact state of their lower qubits
+    if (nstates == 1 && !streamed && nqubits >= qse::kCompactMinQubits && !pl.passes.empty()) {
+        const uint64_t compact = (uint64_t(1) << qse::kCompactMaxQubits) - 1;
+        const qse::plan::Plan first =
+            qse::plan::build(gates, nqubits, perm, qse::plan::forward_options(set, nqubits, true));
+        compile(qse::jit::generate(first.passes[0], 1, true, false, pre_groups, compact, nullptr, compact + 1));
     }
     if (source_bytes) *source_bytes = total;
     QSE_GUARD_END

@@ -351,12 +351,6 @@ __global__ void __launch_bounds__(256) k_group_values(const plan::TermRec* __res
     }
 }
 
-uint32_t tile_qubits_for(const qse_ctx* ctx, uint32_t n, uint32_t rb, uint32_t kmax)
-{
-    uint32_t k = std::min<uint32_t>(std::max(ctx->tile_qubits, int(rb) + 1), kmax);
-    return std::min(k, n);
-}
-
 // Specialised pass kernels repay their compile time (NVRTC: about a second or
 // more per distinct kernel) when a pass is expensive, i.e. on large states, or
 // when few of a plan's kernels are new.  A deep circuit on a small state can
@@ -367,31 +361,6 @@ uint32_t tile_qubits_for(const qse_ctx* ctx, uint32_t n, uint32_t rb, uint32_t k
 // compilation may cost is counted in the kernels of 12-qubit tiles.
 constexpr uint32_t kJitAlwaysQubits = 22;
 constexpr size_t kJitMaxNewKernels = 32;
-// States of at most kSmallQubits qubits hold 8 amplitudes per thread in tiles of
-// 2^11 (up to kTile11Qubits, where more passes cost more than fuller SMs give)
-// or 2^10: with 32 per thread and 2^12 they are a few CTAs of four warps each
-// (16 at 16 qubits), bound by fetching their straight-line code, a quarter as
-// long with 8 per thread.  Layered rotations, execute and download: 12 qubits
-// 235 -> 114 us, 14 qubits 427 -> 229, 16 qubits 605 -> 348 (tiles of 2^10: 113,
-// 220, 370); on the device, 20 qubits 115 -> 93 (2^11: 105), random layers of 19
-// qubits 67 -> 63 (69).
-constexpr uint32_t kTile11Qubits = 18;
-constexpr uint32_t kSmallQubits = 20;
-// States of at least this many qubits (128 MiB, beyond the L2) plan their layouts
-// for contiguous memory accesses (Options::low_lanes), at the price of a few more
-// layout exchanges: <O> of a 28-qubit QAOA circuit 9.6 -> 7.9 ms, 25-qubit
-// random layers 1.93 -> 1.75 ms, 25-qubit layered rotations 1.18 -> 1.04 ms,
-// 26-qubit H+RZ+QFT 0.74 -> 0.75 ms.  At 22 qubits the exchanges cost more than
-// the accesses (HEA gradient 1.84 -> 1.91 ms).
-constexpr uint32_t kLowLanesQubits = 23;
-// States of at least this many qubits move what is left of the lowest qubits to
-// the lanes by shuffles (Options::lane_swaps).  On top of low_lanes: 28-qubit
-// QAOA energy 8.1 -> 7.6 ms, 24-qubit gradients of a HEA 4.5 -> 4.1 ms and of a
-// QAOA circuit 4.4 -> 4.1 ms; alone (without low_lanes the 28-qubit energy takes
-// 8.5 ms): 22-qubit HEA gradient 1.74 -> 1.69 ms, 20 qubits 0.74 -> 0.72 ms; no
-// gain below.
-constexpr uint32_t kLaneSwapQubits = 20;
-
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
 // compiling, for the interpreter (use_jit = false).
@@ -402,8 +371,6 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
     qse_ctx* ctx = st->ctx;
     auto e = std::make_shared<PlanEntry>();
     e->use_jit = ctx->jit != 0;
-    opt.acc_mul = true;
-    opt.unit_rot = e->use_jit;
     KeyWriter w;
     w.put('F');
     w.put(ctx->jit);
@@ -453,7 +420,7 @@ std::shared_ptr<PlanEntry> plan_for(qse_state* st, const std::vector<plan::Gate>
             plan::Options iopt = opt;
             iopt.rb = ns == 2 ? 3 : 4;   // as the interpreter kernel is instantiated
             iopt.rb_first = 0;
-            if (ns == 1) iopt.k = tile_qubits_for(ctx, st->n, 4, 12);
+            if (ns == 1) iopt.k = plan::tile_size(ctx->tile_qubits, st->n, 4, 12);
             bool interpret = iopt.k == opt.k;
             if (!interpret) {
                 std::vector<jit::Source> full;
@@ -588,30 +555,9 @@ void run_noise(qse_state* st, qse_noise* nz, const qse_op* ops, size_t nops, con
     QSE_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
-plan::Options fused_options(const qse_ctx* ctx, uint32_t n, bool compact_input = false)
+plan::Settings settings(const qse_ctx* ctx)
 {
-    plan::Options opt;
-    opt.rb = 4;
-    opt.k = tile_qubits_for(ctx, n, 4, 12);
-    // A pass that makes its input from a compact state writes memory but does not
-    // read it, and is bound by FP64 and its layout exchanges: 32 amplitudes per
-    // thread (128 threads, three CTAs per SM) take an exchange per five register
-    // qubits and share each phase factor among twice the amplitudes (30-qubit
-    // H+RZ+QFT 5.5 ms, with 16 per thread 6.8).  Passes that read and write
-    // memory hold 16 (256 threads, two CTAs): a third more warps to keep loads in
-    // flight, and half the code to fetch (27-qubit random layers 0.72-0.83 ms a
-    // pass, with 32 per thread 1.12-1.24).
-    if (ctx->jit == 1 && opt.k == 12 && compact_input) opt.rb_first = 5;
-    if (ctx->jit == 1 && ctx->tile_qubits == 12 && !ctx->exact_tiles && n <= kSmallQubits) {
-        opt.k = std::min(n <= kTile11Qubits ? 11u : 10u, n);
-        opt.rb = 3;
-    }
-    opt.max_gates = uint32_t(std::max(0, ctx->max_gates_per_pass));
-    if (ctx->jit && (opt.max_gates == 0 || opt.max_gates > plan::kJitMaxGates)) opt.max_gates = plan::kJitMaxGates;
-    opt.zz_fuse = true;
-    opt.low_lanes = n >= kLowLanesQubits;
-    opt.lane_swaps = n >= kLaneSwapQubits;
-    return opt;
+    return plan::Settings{ctx->jit, ctx->tile_qubits, ctx->exact_tiles, ctx->max_gates_per_pass};
 }
 
 // Forward passes of gates on st through the planner; returns the pass count.
@@ -622,7 +568,8 @@ uint64_t run_fused(qse_state* st, const std::vector<plan::Gate>& gates, bool pro
 {
     qse_ctx* ctx = st->ctx;
     prob_out = prob_out && st->size() >= 4096 && ctx->jit != 0;
-    const std::shared_ptr<PlanEntry> e = plan_for(st, gates, fused_options(ctx, st->n, st->lazy_basis && st->lazy_umask), 1, prob_out);
+    const std::shared_ptr<PlanEntry> e =
+        plan_for(st, gates, plan::forward_options(settings(ctx), st->n, st->lazy_basis && st->lazy_umask), 1, prob_out);
     const plan::Plan& pl = e->pl;
     const bool use_jit = e->use_jit;
     const std::vector<jit::Source>& srcs = e->srcs;
@@ -665,9 +612,6 @@ uint64_t run_fused(qse_state* st, const std::vector<plan::Gate>& gates, bool pro
 // SWAP); an untouched qubit keeps its basis bit through the prefix, so in the
 // prefix's diagonal gates and CNOT controls it is a known 0 or 1: those gates
 // drop, lose that qubit, or become a factor of the whole state (compact_gate).
-constexpr uint32_t kCompactMinQubits = 24;   // full states this large (smaller ones gain little)
-constexpr uint32_t kCompactMaxQubits = 22;   // compact states up to this size
-
 // qubits a gate acts on non-diagonally
 uint64_t gate_nondiag(const plan::Gate& g)
 {
@@ -878,11 +822,10 @@ bool compact_prefix(qse_state* st, const std::vector<plan::Gate>& gates_in, std:
     if (!ctx->jit || !st->lazy_basis || st->lazy_umask || st->n < kCompactMinQubits) return false;
     // the zz rewrite moves gates between slots: apply it first so that the
     // plan's source indices name the gates that run
-    plan::Options opt = fused_options(ctx, st->n);
+    plan::Options opt = plan::forward_options(settings(ctx), st->n, false);
     std::vector<plan::Gate> fused;
     const std::vector<plan::Gate>& gates = plan::fuse_zz(gates_in, fused) ? fused : gates_in;
     opt.zz_fuse = false;
-    opt.acc_mul = true;
     KeyWriter w;
     w.put('C');
     w.put_options(opt);
@@ -1384,19 +1327,7 @@ double adjoint_sweep(qse_state* st, const qse_op* ops, size_t nops, const double
         if (ops[i].param >= 0 && parameterised(ops[i].type)) gid = bucket(ops[i].type, ops[i].param, ops[i].coeff);
         rev.push_back(inverse_gate(ops[i], th, gid));
     }
-    plan::Options opt;
-    opt.k = tile_qubits_for(ctx, st->n, 3, 11);
-    // specialised kernels hold 16 amplitudes of both states per thread: the
-    // register shape of the forward passes (128 threads, three CTAs per SM), half
-    // the barriers of 8 per thread, and a layout exchange per four register
-    // qubits instead of three (passes of a 24-qubit QAOA: 452 -> 373 us)
-    opt.rb = ctx->jit && opt.k == 11 ? 4 : 3;
-    opt.grads = true;
-    opt.max_terms = 512;
-    opt.max_gates = plan::kJitMaxGates;
-    opt.low_lanes = st->n >= kLowLanesQubits;
-    opt.lane_swaps = st->n >= kLaneSwapQubits;
-    const std::shared_ptr<PlanEntry> e = plan_for(st, rev, opt, 2);
+    const std::shared_ptr<PlanEntry> e = plan_for(st, rev, plan::adjoint_options(settings(ctx), st->n), 2);
     const plan::Plan& pl = e->pl;
     Uploaded up = upload_plan(ctx, pl, e->use_jit, e->use_jit && st->n >= jit::kPreGroupQubits);
 

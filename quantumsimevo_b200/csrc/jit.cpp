@@ -1258,11 +1258,26 @@ std::string compile_to_cubin(const std::string& src, std::string& err)
     return bin;
 }
 
+// QSE_JIT_DUMP=<directory>: every source compiled is also written there
+// (<entry point>_<hash of the source>.cu), for reading the generated kernels
+void dump_source(const Source& s)
+{
+    const char* dir = std::getenv("QSE_JIT_DUMP");
+    if (!dir || !*dir) return;
+    char name[64];
+    std::snprintf(name, sizeof(name), "_%016zx.cu", std::hash<std::string>{}(s.code));
+    if (FILE* f = std::fopen((std::string(dir) + "/" + s.name + name).c_str(), "w")) {
+        std::fwrite(s.code.data(), 1, s.code.size(), f);
+        std::fclose(f);
+    }
+}
+
 }  // namespace
 
 size_t compile_only(const Source& s)
 {
     if (!available(nullptr)) fail(QSE_ERR_UNSUPPORTED, "NVRTC unavailable: " + nvrtc().why);
+    dump_source(s);
     std::string err;
     std::string bin = compile_to_cubin(s.code, err);
     if (bin.empty()) fail(QSE_ERR_CUDA, "pass kernel compilation failed: " + err);
@@ -1389,17 +1404,7 @@ std::vector<std::shared_ptr<Kernel>> get_kernels(const std::vector<const Source*
             for (size_t w; (w = next.fetch_add(1)) < todo.size();) bins[w] = compile_to_cubin(srcs[todo[w]]->code, errs[w]);
         });
     for (auto& th : pool) th.join();
-    // QSE_JIT_DUMP=<directory>: every source compiled is also written there
-    // (<entry point>_<hash of the source>.cu), for reading the generated kernels
-    if (const char* dir = std::getenv("QSE_JIT_DUMP"); dir && *dir)
-        for (size_t i : todo) {
-            char name[64];
-            std::snprintf(name, sizeof(name), "_%016zx.cu", std::hash<std::string>{}(srcs[i]->code));
-            if (FILE* f = std::fopen((std::string(dir) + "/" + srcs[i]->name + name).c_str(), "w")) {
-                std::fwrite(srcs[i]->code.data(), 1, srcs[i]->code.size(), f);
-                std::fclose(f);
-            }
-        }
+    for (size_t i : todo) dump_source(*srcs[i]);
     std::lock_guard<std::mutex> lk(g_mu);
     for (size_t w = 0; w < todo.size(); ++w) {
         if (bins[w].empty()) fail(QSE_ERR_CUDA, "pass kernel compilation failed: " + errs[w]);

@@ -803,6 +803,83 @@ void bind_angles(Plan& plan, const std::vector<Gate>& gates, const Options& opt)
     bind_gates(plan, (opt.zz_fuse && fuse_zz(gates, fused)) ? fused : gates, opt);
 }
 
+// States of at most kSmallQubits qubits hold 8 amplitudes per thread in tiles of
+// 2^11 (up to kTile11Qubits, where more passes cost more than fuller SMs give)
+// or 2^10: with 32 per thread and 2^12 they are a few CTAs of four warps each
+// (16 at 16 qubits), bound by fetching their straight-line code, a quarter as
+// long with 8 per thread.  Layered rotations, execute and download: 12 qubits
+// 235 -> 114 us, 14 qubits 427 -> 229, 16 qubits 605 -> 348 (tiles of 2^10: 113,
+// 220, 370); on the device, 20 qubits 115 -> 93 (2^11: 105), random layers of 19
+// qubits 67 -> 63 (69).
+constexpr uint32_t kTile11Qubits = 18;
+constexpr uint32_t kSmallQubits = 20;
+// States of at least this many qubits (128 MiB, beyond the L2) plan their layouts
+// for contiguous memory accesses (Options::low_lanes), at the price of a few more
+// layout exchanges: <O> of a 28-qubit QAOA circuit 9.6 -> 7.9 ms, 25-qubit
+// random layers 1.93 -> 1.75 ms, 25-qubit layered rotations 1.18 -> 1.04 ms,
+// 26-qubit H+RZ+QFT 0.74 -> 0.75 ms.  At 22 qubits the exchanges cost more than
+// the accesses (HEA gradient 1.84 -> 1.91 ms).
+constexpr uint32_t kLowLanesQubits = 23;
+// States of at least this many qubits move what is left of the lowest qubits to
+// the lanes by shuffles (Options::lane_swaps).  On top of low_lanes: 28-qubit
+// QAOA energy 8.1 -> 7.6 ms, 24-qubit gradients of a HEA 4.5 -> 4.1 ms and of a
+// QAOA circuit 4.4 -> 4.1 ms; alone (without low_lanes the 28-qubit energy takes
+// 8.5 ms): 22-qubit HEA gradient 1.74 -> 1.69 ms, 20 qubits 0.74 -> 0.72 ms; no
+// gain below.
+constexpr uint32_t kLaneSwapQubits = 20;
+
+uint32_t tile_size(int tile_qubits, uint32_t n, uint32_t rb, uint32_t kmax)
+{
+    return std::min(std::min<uint32_t>(std::max(tile_qubits, int(rb) + 1), kmax), n);
+}
+
+Options forward_options(const Settings& s, uint32_t n, bool compact_input)
+{
+    Options opt;
+    opt.rb = 4;
+    opt.k = tile_size(s.tile_qubits, n, 4, 12);
+    // A pass that makes its input from a compact state writes memory but does not
+    // read it, and is bound by FP64 and its layout exchanges: 32 amplitudes per
+    // thread (128 threads, three CTAs per SM) take an exchange per five register
+    // qubits and share each phase factor among twice the amplitudes (30-qubit
+    // H+RZ+QFT 5.5 ms, with 16 per thread 6.8).  Passes that read and write
+    // memory hold 16 (256 threads, two CTAs): a third more warps to keep loads in
+    // flight, and half the code to fetch (27-qubit random layers 0.72-0.83 ms a
+    // pass, with 32 per thread 1.12-1.24).
+    if (s.jit == 1 && opt.k == 12 && compact_input) opt.rb_first = 5;
+    if (s.jit == 1 && s.tile_qubits == 12 && !s.exact_tiles && n <= kSmallQubits) {
+        opt.k = std::min(n <= kTile11Qubits ? 11u : 10u, n);
+        opt.rb = 3;
+    }
+    opt.max_gates = uint32_t(std::max(0, s.max_gates_per_pass));
+    if (s.jit && (opt.max_gates == 0 || opt.max_gates > kJitMaxGates)) opt.max_gates = kJitMaxGates;
+    opt.acc_mul = true;
+    opt.unit_rot = s.jit != 0;
+    opt.zz_fuse = true;
+    opt.low_lanes = n >= kLowLanesQubits;
+    opt.lane_swaps = n >= kLaneSwapQubits;
+    return opt;
+}
+
+Options adjoint_options(const Settings& s, uint32_t n)
+{
+    Options opt;
+    opt.k = tile_size(s.tile_qubits, n, 3, 11);
+    // specialised kernels hold 16 amplitudes of both states per thread: the
+    // register shape of the forward passes (128 threads, three CTAs per SM), half
+    // the barriers of 8 per thread, and a layout exchange per four register
+    // qubits instead of three (passes of a 24-qubit QAOA: 452 -> 373 us)
+    opt.rb = s.jit && opt.k == 11 ? 4 : 3;
+    opt.grads = true;
+    opt.max_terms = 512;
+    opt.max_gates = kJitMaxGates;
+    opt.acc_mul = true;
+    opt.unit_rot = s.jit != 0;
+    opt.low_lanes = n >= kLowLanesQubits;
+    opt.lane_swaps = n >= kLaneSwapQubits;
+    return opt;
+}
+
 std::string describe(const Plan& p)
 {
     std::ostringstream os;

@@ -177,6 +177,22 @@ struct Options {
                                  // only through op_angles / term_angles)
 };
 
+// What of a context's settings decides how its states' gates are planned.
+struct Settings {
+    int jit = 1;                 // qse_ctx_set_jit
+    int tile_qubits = 12;        // qse_ctx_set_fusion
+    bool exact_tiles = false;
+    int max_gates_per_pass = 0;
+};
+
+// The options of an n-qubit state's forward passes (compact_input: the first one
+// makes its input from a compact state) and of the adjoint sweep's reverse passes.
+// qse_plan_compile plans with the same, so what it compiles is what runs.
+Options forward_options(const Settings& s, uint32_t n, bool compact_input);
+Options adjoint_options(const Settings& s, uint32_t n);
+// tile qubits of a state for a setting and rb register bits, at most kmax
+uint32_t tile_size(int tile_qubits, uint32_t n, uint32_t rb, uint32_t kmax);
+
 struct Plan {
     std::vector<PassProgram> passes;
     uint32_t perm_final[64];

@@ -35,6 +35,12 @@ struct DevBuf {
     ~DevBuf() { release(); }
 };
 
+// Executes of states this large run their leading passes on a compact state of up
+// to kCompactMaxQubits of their qubits (engine.cu, compact prefix; smaller states
+// gain little).
+constexpr uint32_t kCompactMinQubits = 24;
+constexpr uint32_t kCompactMaxQubits = 22;
+
 struct PlanCache;   // engine.cu: plans of recent executes, reused when a program runs again
 
 // Pinned host staging buffer.
@@ -57,7 +63,7 @@ struct qse_ctx {
     int fusion = 1;
     int jit = 1;             // specialised NVRTC pass kernels (0: generic interpreter kernel,
                              // 2: specialised, with the streamed persistent kernel where it applies)
-    int tile_qubits = 12;    // upper limit (small states take smaller tiles: engine.cu, fused_options)
+    int tile_qubits = 12;    // upper limit (small states take smaller tiles: planner.cpp, forward_options)
     bool exact_tiles = false;   // ... unless this is set
     int max_gates_per_pass = 0;
     int sample_mode = 0;
