@@ -888,10 +888,9 @@ __global__ void __launch_bounds__(kBT, 4) k_cdf_summ(const double* __restrict__ 
 // start 45 8-byte words apart, so 16 threads hit 16 distinct bank pairs)
 constexpr int kChainPer = 9;
 constexpr uint32_t kSpan = uint32_t(kChainPer) * kBT;
-// one buffer of k_cdf_chain: a span of fold records copied from a 16-byte
+// the buffer of k_cdf_chain: a span of fold records copied from a 16-byte
 // aligned start (the records start 0 or 8 bytes in), rounded up to 16 bytes
-constexpr uint32_t kSpanBuf = uint32_t((size_t(kSpan) * sizeof(Summ) + 32) & ~size_t(15));
-constexpr size_t kChainSmem = 2 * size_t(kSpanBuf);
+constexpr size_t kChainSmem = (size_t(kSpan) * sizeof(Summ) + 32) & ~size_t(15);
 // bytes after the fold records that a rounded-up copy may read (the
 // scratch that holds them reserves that much beyond them)
 constexpr size_t kSummSlack = 32;
@@ -910,7 +909,6 @@ __device__ __forceinline__ uint32_t summ_fetch(char* buf, const Summ* summ, uint
     const uint32_t skew = uint32_t(s0 - a0);
     const uint32_t bytes = (cnt * uint32_t(sizeof(Summ)) + skew + 15u) & ~15u;
     const char* src = reinterpret_cast<const char*>(summ) + a0;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier reads of buf before the copy's writes
     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
                  "r"(bytes) : "memory");
     constexpr uint32_t kPiece = 32768;
@@ -937,77 +935,38 @@ __device__ __forceinline__ bool chain_wait(uint64_t* bar, uint32_t parity)
     return false;
 }
 
-// Shared memory of the chain (one CTA) besides the two record buffers.
+// Shared memory of the chain (one CTA) besides the fold records.
 struct ChainShm {
     uint64_t sh[160];
     double stage[kBT * kPad];
     double c;          // the exact running sum
     int slow;
     uint32_t end;
-    __align__(8) uint64_t bar[2];
-    uint32_t skew[2];
-};
-
-// The record buffers and their copies.  Every thread holds the same copy of
-// this state and calls fetch/drain together.
-struct ChainIO {
-    ChainShm& S;
-    char* raw;
-    const Summ* summ;
-    uint32_t pend[2] = {0, 0};             // copy in flight, per buffer
-    uint32_t ph[2] = {0, 0};               // parity of its mbarrier phase
-    uint32_t loaded[2] = {~0u, ~0u};       // first block the buffer holds (or will)
-    uint32_t end[2] = {0, 0};              // and the one after its last
-    __device__ ChainIO(ChainShm& s, char* r, const Summ* sm) : S(s), raw(r), summ(sm) {}
-    __device__ void fetch(uint32_t b, uint32_t from, uint32_t cnt)
-    {
-        if (threadIdx.x == 0) S.skew[b] = summ_fetch(raw + b * kSpanBuf, summ, from, cnt, &S.bar[b]);
-        pend[b] = 1;
-        loaded[b] = from;
-        end[b] = from + cnt;
-    }
-    // waits for buffer b's copy; uniform result (a copy not seen done stays pending)
-    __device__ bool drain(uint32_t b)
-    {
-        bool ok = true;
-        if (pend[b]) ok = chain_wait(&S.bar[b], ph[b]);
-        ok = __syncthreads_and(ok) != 0;
-        if (pend[b] && ok) {
-            ph[b] ^= 1u;
-            pend[b] = 0;
-        }
-        return ok;
-    }
-    __device__ const Summ* rec(uint32_t b) const { return reinterpret_cast<const Summ*>(raw + b * kSpanBuf + S.skew[b]); }
+    __align__(8) uint64_t bar;
+    uint32_t skew;     // where the records begin in their buffer
 };
 
 // The exact running sum over blocks [b_begin, b_end), starting from S.c (the
 // exact sum before b_begin) and leaving the sum after b_end there; writes
-// cin[b_begin, b_end).  Each step takes the next span of up to kSpan blocks
-// (kChainPer consecutive per thread): every block up to the first one without
+// cin[b_begin, b_end).  The fold records of the range, at most kSpan, are in
+// shared memory (recs).  Each step takes the blocks left (kChainPer
+// consecutive per thread): every block up to the first one without
 // a fold on the running sum's binade composes with one block-wide scan, and
 // the step commits the blocks up to the first one whose sum would leave the
 // binade (or the one without a fold).  That block is handled on its own (its
 // fold on the binade it actually starts in, else an exact element-by-element
-// fold) and the next span starts after it.  The fold records of a span arrive
-// in shared memory by bulk copies while the previous span is composed (two
-// buffers; a span that stopped early goes on in the same buffer; records already
-// in buffer 0 for b_begin are used as they are).  A running sum of
+// fold) and the next step starts after it.  A running sum of
 // zero is on the grid of binade -1022 (spacing 2^-1074, shared by the
-// subnormals), where zero and subnormal blocks fold exactly.  False when a
-// bounded wait gave up.
-__device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32_t b_begin, uint32_t b_end,
-                            double* __restrict__ cin, uint32_t& n_span, uint32_t& n_single, uint32_t& n_exact)
+// subnormals), where zero and subnormal blocks fold exactly.
+__device__ void chain_range(ChainShm& S, const Summ* recs, const double* __restrict__ prob, uint32_t b_begin,
+                            uint32_t b_end, double* __restrict__ cin, uint32_t& n_span, uint32_t& n_single,
+                            uint32_t& n_exact)
 {
-    ChainShm& S = io.S;
     const uint32_t t = threadIdx.x;
-    uint32_t base = b_begin, cur = 0;
+    uint32_t base = b_begin;
     while (base < b_end) {
-        if (io.loaded[cur] == ~0u) io.fetch(cur, base, min(kSpan, b_end - base));   // the first span
-        const uint32_t next = io.end[cur], span = next - base;
-        if (next < b_end && io.loaded[cur ^ 1] != next) io.fetch(cur ^ 1, next, min(kSpan, b_end - next));
-        if (!io.drain(cur)) return false;
-        const Summ* rec = io.rec(cur) + (base - io.loaded[cur]);
+        const uint32_t span = b_end - base;
+        const Summ* rec = recs + (base - b_begin);
         const double c = S.c;
         const int e0 = epoch_of(c);
         const uint32_t p0 = t * kChainPer;           // this thread's first position in the span
@@ -1062,12 +1021,8 @@ __device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32
             if (pos + 1 == end) S.c = ldexp(double(xin[k] + ((xin[k] & 1) ? d1[k] : d0[k])), e0 - 52);
         }
         if (t == 0 && end > 0) ++n_span;
-        __syncthreads();   // every thread is done with rec and S.c before either changes
-        if (end >= span) {
-            base = next;
-            cur ^= 1;   // fetched above
-            continue;
-        }
+        __syncthreads();   // every thread is done with S.c and S.end before either changes
+        if (end >= span) return;
         // block b starts in the running sum's binade but has no fold there or leaves it
         ++n_single;
         const uint32_t b = base + end;
@@ -1097,9 +1052,7 @@ __device__ bool chain_range(ChainIO& io, const double* __restrict__ prob, uint32
         }
         __syncthreads();
         base = b + 1;
-        if (base == next) cur ^= 1;
     }
-    return true;
 }
 
 // hand-off between consecutive segments of the chain: the exact sum after a
@@ -1140,8 +1093,7 @@ __global__ void __launch_bounds__(kBT, 1) k_cdf_chain(const double* __restrict__
     __shared__ int s_fail;
     const uint32_t t = threadIdx.x;
     if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.bar[0])) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.bar[1])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_seg = atomicAdd(ticket, 1u);
         s_done = 0;
@@ -1150,13 +1102,12 @@ __global__ void __launch_bounds__(kBT, 1) k_cdf_chain(const double* __restrict__
     __syncthreads();
     const uint32_t j = s_seg;
     const uint32_t b0 = j * kSpan, b1 = min(nb, b0 + kSpan), cnt = b1 - b0;
-    ChainIO io(S, sraw, summ);
     uint32_t n_span = 0, n_single = 0, n_exact = 0;
-    io.fetch(0, b0, cnt);
-    bool ok = io.drain(0);
+    if (t == 0) S.skew = summ_fetch(sraw, summ, b0, cnt, &S.bar);
+    bool ok = __syncthreads_and(chain_wait(&S.bar, 0u)) != 0;
+    const Summ* rec = reinterpret_cast<const Summ*>(sraw + S.skew);
     if (ok && j > 0) {
         // the segment's fold on each binade its first block may start in
-        const Summ* rec = io.rec(0);
         const int32_t eg = rec[0].e;
         for (int kb = 0; kb < 2; ++kb) {
             const int e = eg + kb;
@@ -1225,19 +1176,18 @@ __global__ void __launch_bounds__(kBT, 1) k_cdf_chain(const double* __restrict__
     }
     __syncthreads();
     // the segment's own block starts from the exact incoming sum
-    if (ok) ok = chain_range(io, prob, b0, b1, cin, n_span, n_single, n_exact);
-    if (ok && t == 0 && !s_done) {
-        link[j].value = S.c;
-        __threadfence();
-        *(volatile uint32_t*)&link[j].flag = 1u;
-    }
-    // no copy may still be writing shared memory when the CTA leaves
-    const bool dr0 = io.drain(0), dr1 = io.drain(1);
-    if (!ok || !dr0 || !dr1) {
+    if (!ok) {
+        chain_wait(&S.bar, 0u);   // the copy may still be writing shared memory: bounded, like every wait here
         if (t == 0) *(volatile unsigned*)status = 4u;
         return;
     }
+    chain_range(S, rec, prob, b0, b1, cin, n_span, n_single, n_exact);
     if (t == 0) {
+        if (!s_done) {
+            link[j].value = S.c;
+            __threadfence();
+            *(volatile uint32_t*)&link[j].flag = 1u;
+        }
         if (b1 == nb) cin[nb] = S.c;
         if (stats) {
             atomicAdd(stats + 0, n_span);
