@@ -568,7 +568,6 @@ void build(qse_batch* b)
         opt.max_terms = 512;
         opt.keep_gphase = false;
         opt.direct_phases = true;
-        opt.acc_mul = true;
         opt.max_slots = cf.grad_slots;
         uint32_t perm0[64];
         for (uint32_t q = 0; q < 64; ++q) perm0[q] = q;

@@ -85,7 +85,7 @@ struct KeyWriter {
     void put_options(const plan::Options& o)
     {
         put(o.k); put(o.rb); put(o.rb_first); put(o.max_gates); put(o.max_terms); put(o.grads); put(o.max_slots);
-        put(o.direct_phases); put(o.acc_mul); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.lane_swaps); put(o.keep_gphase);
+        put(o.direct_phases); put(o.zz_fuse); put(o.unit_rot); put(o.low_lanes); put(o.lane_swaps); put(o.keep_gphase);
     }
     // everything but the angles and the matrices
     void put_gates(const std::vector<plan::Gate>& gates)
@@ -291,12 +291,12 @@ Uploaded upload_plan(qse_ctx* ctx, const plan::Plan& pl, bool specialised, bool 
 }
 
 // The per-CTA values of a pass's diagonal groups, one row per tile (out[t * ng
-// + g], the row CTA t of the pass copies).  The value of a direct group is the
+// + g], the row CTA t of the pass copies).  The value of a group is the
 // product of the unit phases (cos, sin) of its terms whose outer-qubit
 // conditions hold for t's outer bits (t's bits deposited on the outer positions
 // in ascending order, as the pass kernel numbers its CTAs); each term's phase
 // is computed once on the host, so this kernel multiplies and never takes a
-// sincos.  Other groups keep the plain sum of their angles.  A CTA handles
+// sincos.  A CTA handles
 // kGvTiles consecutive tiles: their outer bits once into shared memory, then
 // its threads walk the rows' elements in address order (coalesced stores).
 // For the two tables of a split pass (jit::Source::gv_lo) the "tiles" are the
@@ -329,23 +329,13 @@ __global__ void __launch_bounds__(256) k_group_values(const plan::TermRec* __res
         const uint32_t tl = e / ng, g = e - tl * ng;
         const uint64_t ob = s_ob[tl];
         const plan::GroupRec gr = groups[g];
-        double2 v;
-        if (gr.direct) {
-            v = make_double2(1.0, 0.0);
-            for (uint32_t k = 0; k < gr.count; ++k) {
-                const uint64_t oc = terms[gr.first + k].ocond;
-                if ((ob & oc) == oc && (oc || !skip_unconditioned)) {
-                    const double2 f = texp[gr.first + k];
-                    v = make_double2(v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
-                }
+        double2 v = make_double2(1.0, 0.0);
+        for (uint32_t k = 0; k < gr.count; ++k) {
+            const uint64_t oc = terms[gr.first + k].ocond;
+            if ((ob & oc) == oc && (oc || !skip_unconditioned)) {
+                const double2 f = texp[gr.first + k];
+                v = make_double2(v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
             }
-        } else {
-            double th = 0.0;
-            for (uint32_t k = 0; k < gr.count; ++k) {
-                const plan::TermRec t = terms[gr.first + k];
-                if ((ob & t.ocond) == t.ocond && (t.ocond || !skip_unconditioned)) th += t.theta;
-            }
-            v = make_double2(th, 0.0);
         }
         row[e] = v;
     }
@@ -361,6 +351,7 @@ __global__ void __launch_bounds__(256) k_group_values(const plan::TermRec* __res
 // compilation may cost is counted in the kernels of 12-qubit tiles.
 constexpr uint32_t kJitAlwaysQubits = 22;
 constexpr size_t kJitMaxNewKernels = 32;
+
 // Plans gates for the specialised kernels (their sources generated into srcs,
 // use_jit = true) or, when the context disables them or they are not worth
 // compiling, for the interpreter (use_jit = false).

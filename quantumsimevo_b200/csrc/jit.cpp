@@ -306,31 +306,7 @@ struct Gen {
         }
     }
 
-    void emit_flush_reg(int p)
-    {
-        if (P.acc_mul) {
-            o << "  if (notOne(ar" << p << ")) { const double2 e = ar" << p << "; ar" << p
-              << " = make_double2(1.0, 0.0);";
-        } else {
-            o << "  if (ar" << p << " != 0.0) { const double2 e = expi(ar" << p << "); ar" << p << " = 0.0;";
-        }
-        for (int s = 0; s < ns; ++s) o << " phD<" << (1 << p) << ">(" << (s ? "a1" : "a0") << ", e);";
-        o << " }\n";
-    }
-
-    // per-thread accumulators: angles (sincos at each flush) or, with acc_mul,
-    // complex factors multiplied by the groups' per-CTA (cos, sin)
-    void emit_acc_decls()
-    {
-        const char* ty = P.acc_mul ? "double2" : "double";
-        const char* one = P.acc_mul ? "make_double2(1.0, 0.0)" : "0.0";
-        o << "  " << ty << " at = " << one;
-        for (uint32_t i = 0; i < P.rb; ++i) o << ", ar" << i << " = " << one;
-        o << ";\n";
-        for (uint32_t i = P.rb; i < 5; ++i) o << "  " << ty << " ar" << i << " = " << one << "; (void)ar" << i << ";\n";
-    }
-
-    // ---- acc_mul: merged diagonal runs ----
+    // ---- merged diagonal runs ----
     // Diagonal ops between two non-diagonal ones commute.  Each run becomes
     // one factor per register mask M (the product of its K_PHD groups, its
     // flushed accumulator chain, or, for M = 0, the K_ACC_THR chain times the
@@ -343,10 +319,10 @@ struct Gen {
     struct Item { uint16_t tcond; uint16_t g; };
     struct Fac { std::vector<Item> items; std::vector<uint32_t> consts; };   // consts: K_FLUSH_ALL ops
     static constexpr uint32_t kMaxTables = 32;
-    static constexpr int kThrChain = 5;   // chain index of the thread accumulator (after ar0..ar4)
+    static constexpr int kThrChain = 5;   // chain index of the thread accumulator (after the five register bits)
     uint32_t max_tables = kMaxTables;   // 0 with precomputed group values (no prologue)
     std::vector<uint32_t> run_ops;   // indices into P.ops
-    std::vector<Item> chain[kThrChain + 1];   // pending accumulator groups: ar0..ar4, at
+    std::vector<Item> chain[kThrChain + 1];   // pending accumulator groups: register bits 0..4, thread
     std::ostringstream tabs;      // prologue code building the lane tables
     uint32_t ntab = 0;
     uint32_t nvar = 0;
@@ -359,15 +335,13 @@ struct Gen {
 
     void emit_op(const plan::KOp& op)
     {
-        if (P.acc_mul) {
-            if (diag_kind(op.kind)) { run_ops.push_back(uint32_t(&op - P.ops.data())); return; }
-            if (op.kind == plan::K_GRAD_Z || op.kind == plan::K_GRAD_P) {
-                if (!run_unimodular()) flush_run();
-                add_phase_grad(op);
-                return;
-            }
-            flush_run();
+        if (diag_kind(op.kind)) { run_ops.push_back(uint32_t(&op - P.ops.data())); return; }
+        if (op.kind == plan::K_GRAD_Z || op.kind == plan::K_GRAD_P) {
+            if (!run_unimodular()) flush_run();
+            add_phase_grad(op);
+            return;
         }
+        flush_run();
         emit(op);
     }
 
@@ -581,7 +555,6 @@ struct Gen {
         set_layout(P.layouts[P.layout0]);
         std::ostringstream body;
         std::swap(o, body);
-        if (!P.acc_mul) emit_acc_decls();
         for (const plan::KOp& op : P.ops) emit_op(op);
         flush_run();
         // store (final layout, its lowest qubits moved to the lanes)
@@ -722,19 +695,9 @@ struct Gen {
               << ld("gvt", hex(rows_lo * ng) + " + (u64)(blockIdx.x >> " + std::to_string(gv_lo) + ") * " +
                                std::to_string(ng) + "u + g", total)
               << ";\n";
-            // the groups' kinds are known here: no load of the group records.  The
-            // product's roundings are written out (no contraction left to the
+            // the product's roundings are written out (no contraction left to the
             // compiler), so the debug mode's kernel gives the same bits
-            bool all_direct = true, none_direct = true;
-            for (const plan::GroupRec& gr : P.groups) {
-                all_direct = all_direct && gr.direct;
-                none_direct = none_direct && !gr.direct;
-            }
-            const std::string prod = "make_double2(__fma_rn(l.x, h.x, -__dmul_rn(l.y, h.y)), __fma_rn(l.x, h.y, __dmul_rn(l.y, h.x)))";
-            const std::string sum = "make_double2(__dadd_rn(l.x, h.x), 0.0)";
-            if (all_direct) o << "    gv[g] = " << prod << ";\n  }\n";
-            else if (none_direct) o << "    gv[g] = " << sum << ";\n  }\n";
-            else o << "    gv[g] = groups[g].direct ? " << prod << " : " << sum << ";\n  }\n";
+            o << "    gv[g] = make_double2(__fma_rn(l.x, h.x, -__dmul_rn(l.y, h.y)), __fma_rn(l.x, h.y, __dmul_rn(l.y, h.x)));\n  }\n";
         } else if (ng && pre_gv) {
             o << "  for (u32 g = tid; g < " << ng << "u; g += " << T << "u) gv[g] = "
               << ld("gvt", "(u64)blockIdx.x * " + std::to_string(ng) + "u + g", "(u64)gridDim.x * " + std::to_string(ng) + "u")
@@ -754,7 +717,7 @@ struct Gen {
               << "    const GroupRec gr = groups[g]; double th = 0.0;\n"
               << "    for (u32 i = 0; i < gr.count; ++i) { const TermRec t = " << (stage ? "ts" : "terms")
               << "[gr.first + i]; if ((ob & t.ocond) == t.ocond) th += t.theta; }\n"
-              << "    gv[g] = gr.direct ? expi(th) : make_double2(th, 0.0);\n  }\n";
+              << "    gv[g] = expi(th);\n  }\n";
         }
         if (ntab) o << "  __syncthreads();\n" << tabs.str();
         if (ns == 2 && nslots) o << "  for (u32 i = tid; i < " << nslots * NW << "u; i += " << T << "u) wp[i] = 0.0;\n";
@@ -1000,7 +963,6 @@ struct Gen {
         set_layout(P.layouts[P.layout0]);
         std::ostringstream body;
         std::swap(o, body);
-        if (!P.acc_mul) emit_acc_decls();
         for (const plan::KOp& op : P.ops) emit_op(op);
         flush_run();
         o << "      gb = " << gbase_expr() << ";\n";
@@ -1070,7 +1032,7 @@ struct Gen {
               << "      const GroupRec gr = groups[g]; double th = 0.0;\n"
               << "      for (u32 i = 0; i < gr.count; ++i) { const TermRec t = ts[gr.first + i];"
                  " if ((ob & t.ocond) == t.ocond) th += t.theta; }\n"
-              << "      gv[g] = gr.direct ? expi(th) : make_double2(th, 0.0);\n    }\n";
+              << "      gv[g] = expi(th);\n    }\n";
             s << "    " << SYNC << "\n";
             if (ntab) s << tabs.str() << "    " << SYNC << "\n";
         }
@@ -1141,49 +1103,6 @@ struct Gen {
             guarded("opU<" + std::to_string(p) + ", " + std::to_string(op.f) + ">(@A, &P.v[" + std::to_string(i) + "]);");
             break;
         }
-        case K_ACC_THR:
-            o << "  " << (op.tcond ? "if (" + cond(op.tcond, 0) + ") " : std::string());
-            if (P.acc_mul) o << "at = cmul(at, gv[" << op.g << "]);\n";
-            else o << "at += gv[" << op.g << "].x;\n";
-            break;
-        case K_ACC_REG:
-            o << "  " << (op.tcond ? "if (" + cond(op.tcond, 0) + ") " : std::string());
-            if (P.acc_mul) o << "ar" << p << " = cmul(ar" << p << ", gv[" << op.g << "]);\n";
-            else o << "ar" << p << " += gv[" << op.g << "].x;\n";
-            break;
-        case K_PHD: {
-            std::string t = op.tcond ? "if (" + cond(op.tcond, 0) + ") " : std::string();
-            o << "  " << t << "{ const double2 e = gv[" << op.g << "];";
-            for (int s = 0; s < ns; ++s) o << " phD<" << int(op.f) << ">(" << (s ? "a1" : "a0") << ", e);";
-            o << " }\n";
-            break;
-        }
-        case K_FLUSH_REG: emit_flush_reg(p); break;
-        case K_FLUSH_ALL: {
-            for (uint32_t r = 0; r < P.rb; ++r)
-                if ((op.f >> r) & 1) emit_flush_reg(int(r));
-            const bool unit = op.q == 0;
-            if (P.acc_mul) {
-                if (unit) {
-                    o << "  if (notOne(at)) { const double2 e = at; at = make_double2(1.0, 0.0);";
-                } else {
-                    uint32_t i = push_op(op, Source::PrmRef::op_a);
-                    push_op(op, Source::PrmRef::op_b);
-                    o << "  { const double2 e = cmul(make_double2(P.v[" << i << "], P.v[" << i + 1
-                      << "]), at); at = make_double2(1.0, 0.0);";
-                }
-            } else if (unit) {
-                o << "  if (at != 0.0) { const double2 e = expi(at); at = 0.0;";
-            } else {
-                uint32_t i = push_op(op, Source::PrmRef::op_a);
-                push_op(op, Source::PrmRef::op_b);
-                o << "  { double2 e = make_double2(P.v[" << i << "], P.v[" << i + 1 << "]);"
-                  << " if (at != 0.0) { e = cmul(e, expi(at)); at = 0.0; }";
-            }
-            for (int s = 0; s < ns; ++s) o << " scaleAll(" << (s ? "a1" : "a0") << ", e);";
-            o << " }\n";
-            break;
-        }
         case K_TRANSPOSE: {
             const LayoutRec& nl = P.layouts[op.g];
             o << "  {\n    const u32 sw = " << slot_expr(nl) << ";\n";
@@ -1204,7 +1123,7 @@ struct Gen {
             o << "  }\n";
             break;
         }
-        case K_GRAD_X: case K_GRAD_Y:
+        case K_GRAD_X: case K_GRAD_Y:   // (emit_op has the other two, and every diagonal op)
             if (ns == 2)
                 add_to_slot(op.g, (op.kind == K_GRAD_X ? "gradX<" : "gradY<") + std::to_string(p) + ">(a0, a1)",
                             push_op(op, Source::PrmRef::op_a));

@@ -39,7 +39,7 @@ struct Source {
     // gv_lo outer qubits or in the others, so the table is two tables: one row
     // per value of the low gv_lo CTA-index bits, then one per value of the
     // other bits (terms without a condition in the first only); a CTA's value
-    // is the product (direct groups) or the sum (angle groups) of its two rows'
+    // is the product of its two rows'
     uint32_t gv_lo = 0;
 };
 

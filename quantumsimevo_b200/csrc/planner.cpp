@@ -459,9 +459,9 @@ private:
         split(sup, f, tc, oc);
         int nreg = popc(f);
         // direct_phases: terms on register bits whose angle does not depend on
-        // the thread (no thread condition) are direct, their group's sum turned
-        // into (cos, sin) once per CTA; otherwise single-bit terms accumulate
-        // angles per thread, one sincos per flush.
+        // the thread (no thread condition) multiply the registers at once;
+        // otherwise single-bit terms multiply into a phase per thread and bit,
+        // applied at the bit's flush.
         const bool direct1 = opt_.direct_phases && tc == 0;
         int kind = nreg == 0 ? K_ACC_THR : ((nreg == 1 && !direct1) ? K_ACC_REG : K_PHD);
         int key2 = kind == K_ACC_REG ? __builtin_ctz(f) : (kind == K_PHD ? f : 0);
@@ -494,7 +494,6 @@ private:
         GroupRec gr{};
         gr.first = uint32_t(P.terms.size());
         gr.count = uint32_t(og.terms.size());
-        gr.direct = (og.kind == K_PHD || opt_.acc_mul) ? 1u : 0u;
         for (size_t i = 0; i < og.src.size(); ++i)
             if (og.src[i] >= 0) P.term_angles.push_back(AngleRef{uint32_t(P.terms.size() + i), uint32_t(og.src[i])});
         P.terms.insert(P.terms.end(), og.terms.begin(), og.terms.end());
@@ -775,7 +774,6 @@ Plan build(const std::vector<Gate>& gates_in, uint32_t n, const uint32_t* perm_i
         PassProgram prog;
         prog.k = k;
         prog.rb = plan.passes.empty() && opt.rb_first ? opt.rb_first : opt.rb;
-        prog.acc_mul = opt.acc_mul;
         prog.lane_swaps = opt.lane_swaps;
         uint32_t b = 0;
         for (uint32_t q = 0; q < n; ++q)
@@ -853,7 +851,6 @@ Options forward_options(const Settings& s, uint32_t n, bool compact_input)
     }
     opt.max_gates = uint32_t(std::max(0, s.max_gates_per_pass));
     if (s.jit && (opt.max_gates == 0 || opt.max_gates > kJitMaxGates)) opt.max_gates = kJitMaxGates;
-    opt.acc_mul = true;
     opt.unit_rot = s.jit != 0;
     opt.zz_fuse = true;
     opt.low_lanes = n >= kLowLanesQubits;
@@ -873,7 +870,6 @@ Options adjoint_options(const Settings& s, uint32_t n)
     opt.grads = true;
     opt.max_terms = 512;
     opt.max_gates = kJitMaxGates;
-    opt.acc_mul = true;
     opt.unit_rot = s.jit != 0;
     opt.low_lanes = n >= kLowLanesQubits;
     opt.lane_swaps = n >= kLaneSwapQubits;

@@ -29,11 +29,11 @@ enum KKind : uint8_t {
                    // where |c| >= |s|, else by s, (a,b) = (c/s, 0) (the pass scale carries the divisor)
     K_RY,          // [[c,-s],[s,c]] on p, likewise
     K_U,           // generic 2x2 on p, matrix index g, controls as K_X
-    K_ACC_THR,     // if thread cond: acc_thr += group value g  (acc_mul: acc_thr *= (cos, sin) g)
-    K_ACC_REG,     // if thread cond: acc[p] += group value g   (acc_mul: acc[p] *= (cos, sin) g)
-    K_PHD,         // if thread cond: amplitudes with (j & f) == f *= group (cos, sin) g
-    K_FLUSH_REG,   // amplitudes with bit p *= e^{i acc[p]}; acc[p] = 0
-    K_FLUSH_ALL,   // flush acc[p] for p in f, then all amplitudes *= e^{i acc_thr} * (a + ib);
+    K_ACC_THR,     // if thread cond: acc_thr *= group value g
+    K_ACC_REG,     // if thread cond: acc[p] *= group value g
+    K_PHD,         // if thread cond: amplitudes with (j & f) == f *= group value g
+    K_FLUSH_REG,   // amplitudes with bit p *= acc[p]; acc[p] = 1
+    K_FLUSH_ALL,   // flush acc[p] for p in f, then all amplitudes *= acc_thr * (a + ib);
                    // q: 0 = the constant is 1, 1 = it has modulus 1, 2 = any
     K_TRANSPOSE,   // exchange through shared memory into layout g
     K_GRAD_X,      // slot g += sum_pairs Im(conj(l0) s1 + conj(l1) s0)         (RX generator)
@@ -80,11 +80,9 @@ struct TermRec {       // one diagonal term: angle theta if all outer bits of oc
     double theta;
 };
 
-struct GroupRec {      // terms [first, first+count) summed per CTA; direct groups get (cos, sin)
+struct alignas(8) GroupRec {   // terms [first, first+count): value (cos, sin) of their angles' sum, per CTA
     uint32_t first;
     uint32_t count;
-    uint32_t direct;
-    uint32_t pad;
 };
 
 // An angle-carrying record of a pass and the source gate it came from: a
@@ -98,7 +96,6 @@ struct AngleRef {
 struct PassProgram {
     uint32_t k = 0;                 // tile qubits
     uint32_t rb = 4;                // register bits per thread
-    bool acc_mul = false;           // accumulators carry complex factors (Options::acc_mul)
     bool lane_swaps = false;        // Options::lane_swaps
     uint64_t outer_mask = 0;        // physical qubits not in the tile
     uint8_t tile_phys[16] = {0};    // physical qubit of tile-local bit b (ascending)
@@ -160,13 +157,10 @@ struct Options {
     bool grads = false;          // emit K_GRAD_* for gates with grad >= 0
     uint32_t max_slots = 0;      // gradient slots per pass, 0 = no cap
     bool direct_phases = false;  // single-register-bit phase terms without a thread
-                                 // condition as direct (cos, sin) groups
-    bool acc_mul = false;        // accumulator groups (K_ACC_THR / K_ACC_REG) are direct too:
-                                 // kernels multiply their (cos, sin) into per-thread complex
-                                 // factors instead of summing angles and calling sincos per flush
+                                 // condition as K_PHD, not through an accumulator
     bool zz_fuse = false;        // rewrite CNOT(c,t) RZ(th,t) CNOT(c,t) as the diagonal
                                  // RZ(th,c) PHASE(th,t) CPHASE(-2th,c,t) (same three slots;
-                                 // only for plans whose angles are never rebound)
+                                 // bind_angles rewrites the new gates likewise)
     bool lane_swaps = false;     // specialised kernels move physical qubits 0..2 from the registers to the
                                  // lanes by shuffles where a pass reads and writes
     bool low_lanes = false;      // the layouts keep physical qubits 0..2 out of the registers where a pass reads and writes
@@ -196,7 +190,6 @@ uint32_t tile_size(int tile_qubits, uint32_t n, uint32_t rb, uint32_t kmax);
 struct Plan {
     std::vector<PassProgram> passes;
     uint32_t perm_final[64];
-    double gphase = 0.0;         // global phase (RZ's e^{-i theta/2}), folded into the last pass
     uint64_t gates = 0;
 };
 

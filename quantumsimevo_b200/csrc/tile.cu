@@ -141,7 +141,6 @@ void launch_pass(qse_ctx* ctx, const PassArgs& a, uint32_t n, uint32_t rb, int n
     if (rb == 4 && nstates == 1) launch_t<4, 1, 8>(ctx, a, n, smem);
     else if (rb == 3 && nstates == 2 && few) launch_t<3, 2, 1>(ctx, a, n, smem);
     else if (rb == 3 && nstates == 2) launch_t<3, 2, 8>(ctx, a, n, smem);
-    else if (rb == 3 && nstates == 1) launch_t<3, 1, 8>(ctx, a, n, smem);
     else fail(QSE_ERR_INVALID, "unsupported tile configuration");
 }
 
