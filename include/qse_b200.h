@@ -320,7 +320,9 @@ QSE_API int qse_batch_total_params(const qse_batch* b, size_t* n);
  * fused per pass, how many tiles a circuit may have and still run start to end
  * in one CTA) with the parameters of the last run (zeros before the first) and
  * keeps the fastest.  cache_path (may be NULL): a JSON file of earlier results,
- * keyed by the batch's structure and the device; read first, updated after. */
+ * keyed by the batch's structure, the device and a revision of the batched
+ * kernels (what was measured on earlier ones is not used); read first, updated
+ * after. */
 QSE_API int qse_batch_autotune(qse_batch* b, const char* cache_path);
 /* 1 (default): every run replays one CUDA graph [reset counters, bind angles,
  * persistent kernel, reductions]; 0: the same launches issued one by one. */
@@ -338,7 +340,8 @@ typedef struct qse_batch_config {
     uint32_t ctas_per_sm;   /* persistent CTAs per SM, 0 = as many as fit                 */
     uint32_t grad_slots;    /* gradient slots per pass, 0 = no cap                        */
     uint32_t wide_regs;     /* 1: up to 255 registers per thread (threads <= 256); 0: 128,
-                               or 168 with 16 amplitudes per thread                       */
+                               or 168 with 16 amplitudes per thread, but up to 255 with
+                               threads 512 and reg_bits 3 (CTAs of 256 threads)           */
 } qse_batch_config;
 QSE_API int qse_batch_set_config(qse_batch* b, const qse_batch_config* cfg);
 /* Bound of the persistent kernel's dependency waits: a work item polls the

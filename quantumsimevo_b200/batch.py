@@ -28,7 +28,8 @@ class BatchConfig:
     chain_tiles: int = 1    # circuits with <= this many tiles run start to end in one CTA
     ctas_per_sm: int = 0    # 0 = as many as fit
     grad_slots: int = 0     # gradient slots per pass, 0 = no cap
-    wide_regs: int = 0      # 1: up to 255 registers per thread (threads <= 256); 0: 128
+    wide_regs: int = 0      # 1: up to 255 registers per thread (threads <= 256); 0: 128, 168 with 16 amplitudes
+                            # per thread, and up to 255 with threads 512 and reg_bits 3
 
 
 class Batch:

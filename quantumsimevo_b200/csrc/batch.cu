@@ -938,6 +938,11 @@ void check_ctl(qse_batch* b)
                                   " (bounded wait gave up; results are invalid)");
 }
 
+// What a configuration stands for: raised when shape_of, the kernels or the rules
+// of the work queue change, so that a cache file's measurements of earlier ones
+// are taken again.
+constexpr uint64_t kConfigRevision = 2;
+
 std::string signature(const qse_batch* b)
 {
     uint64_t h = 1469598103934665603ull;
@@ -947,6 +952,7 @@ std::string signature(const qse_batch* b)
             h *= 1099511628211ull;
         }
     };
+    mix(kConfigRevision);
     mix(b->circs.size());
     for (const CircuitHost& c : b->circs) {
         mix(c.w);
