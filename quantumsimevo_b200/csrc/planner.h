@@ -129,6 +129,8 @@ struct PassProgram {
     std::vector<uint32_t> gphase_src;
     std::vector<uint32_t> mat_src;
     bool deferred = false;          // the pass constant goes to the next pass instead of the last flush
+    // SWAPs only, and no constant to apply: the output is the input
+    bool idle() const { return n_nondiag == 0 && groups.empty() && slot_src.empty() && (ops.empty() || ops.back().q == 0); }
 };
 
 // ---- planner input ----
