@@ -1009,26 +1009,27 @@ namespace {
 
 constexpr int kRB = 256;
 
-// O(x) for the 2^kObsBits amplitudes of a thread, which differ in index bits
-// kObsLow .. kObsLow + kObsBits - 1.  A term's sign splits into the parity of
+// O(x) for the 2^BITS amplitudes of a thread, which differ in index bits
+// kObsLow .. kObsLow + BITS - 1.  A term's sign splits into the parity of
 // the thread's own bits and that of those register bits, so each term adds its
 // signed weight once per thread to the coefficient of its register pattern
 // (the terms come sorted by pattern, first[] = where each begins), and a
-// Walsh-Hadamard transform of the 16 coefficients gives the 16 values.
-constexpr uint32_t kObsBits = 4;
+// Walsh-Hadamard transform of the 2^BITS coefficients gives the values.
+constexpr uint32_t kObsBits = 4;     // on large states
 constexpr uint32_t kObsLow = 8;      // kRB = 2^kObsLow threads hold the bits below
-constexpr int kObsR = 1 << kObsBits;
 constexpr size_t kObsMaxTerms = 4096;   // 64 KiB of shared memory: two CTAs still fit on an SM
 struct ObsFirst {
-    uint16_t first[kObsR + 1];
+    uint16_t first[(1 << kObsBits) + 1];
 };
 
 // partial[b] = sum O(x)|psi_x|^2 over the block's share; lam = O psi if lam !=
-// nullptr.  A CTA takes chunks of 4096 consecutive amplitudes, 16 per thread
-// (two CTAs per SM hold 128 KiB of loads in flight).  Bound by HBM (16 B per
+// nullptr.  A CTA takes chunks of 4096 consecutive amplitudes, 16 per thread (BITS 4;
+// two CTAs per SM hold 128 KiB of loads in flight).  Bound by HBM (16 B per
 // amplitude, 32 with lam).  At 28 qubits and 42 terms an expectation takes 4.5 ms
 // less than with one loop over the terms per amplitude (<O> of a QAOA circuit,
-// execute included: 15.4 -> 11.0 ms).
+// execute included: 15.4 -> 11.0 ms).  Small states take BITS 0, an amplitude per
+// thread (launch_obs).
+template <uint32_t BITS>
 __global__ void __launch_bounds__(kRB, 2) k_obs(const double2* __restrict__ psi, double2* __restrict__ lam, uint64_t size,
                                                 const uint64_t* __restrict__ z, const double* __restrict__ w, uint32_t nt,
                                                 const __grid_constant__ ObsFirst f, double c, double* __restrict__ partial)
@@ -1039,9 +1040,11 @@ __global__ void __launch_bounds__(kRB, 2) k_obs(const double2* __restrict__ psi,
     for (uint32_t t = threadIdx.x; t < nt; t += blockDim.x) { sz[t] = z[t]; sw[t] = w[t]; }
     __syncthreads();
     double acc = 0.0;
+    constexpr int kObsR = 1 << BITS;
     constexpr uint64_t kChunk = uint64_t(kRB) * kObsR;
     for (uint64_t base = blockIdx.x * kChunk; base < size; base += gridDim.x * kChunk) {
         const uint64_t i0 = base + threadIdx.x;
+        if (i0 >= size) continue;   // fewer amplitudes than threads
         double2 v[kObsR];
 #pragma unroll
         for (int j = 0; j < kObsR; ++j) {
@@ -1131,7 +1134,7 @@ struct ObsDev {
 
 // Physical-qubit copy of the observable in device scratch (after `reserve_extra`
 // bytes), its terms sorted by their register pattern (k_obs).
-ObsDev upload_obs(qse_state* st, const qse_observable* obs, char* dbase, char* hbase)
+ObsDev upload_obs(qse_state* st, const qse_observable* obs, uint32_t bits, char* dbase, char* hbase)
 {
     ObsDev o{};
     o.nt = uint32_t(obs->nterms);
@@ -1139,8 +1142,9 @@ ObsDev upload_obs(qse_state* st, const qse_observable* obs, char* dbase, char* h
     uint64_t* hz = reinterpret_cast<uint64_t*>(hbase);
     double* hw = reinterpret_cast<double*>(hbase + 8 * obs->nterms);
     std::vector<uint64_t> phys(obs->nterms);
-    uint32_t count[kObsR] = {0};
-    auto pattern = [](uint64_t m) { return uint32_t(m >> kObsLow) & uint32_t(kObsR - 1); };
+    const uint32_t patterns = 1u << bits;
+    uint32_t count[1 << kObsBits] = {0};
+    auto pattern = [&](uint64_t m) { return uint32_t(m >> kObsLow) & (patterns - 1); };
     for (size_t t = 0; t < obs->nterms; ++t) {
         uint64_t m = obs->zmask[t], pm = 0;
         if (st->n < 64 && (m >> st->n) != 0) fail(QSE_ERR_QUBIT, "observable acts on a qubit out of range");
@@ -1148,8 +1152,8 @@ ObsDev upload_obs(qse_state* st, const qse_observable* obs, char* dbase, char* h
         phys[t] = pm;
         ++count[pattern(pm)];
     }
-    uint32_t at[kObsR];
-    for (int p = 0; p < kObsR; ++p) {
+    uint32_t at[1 << kObsBits];
+    for (uint32_t p = 0; p < patterns; ++p) {
         at[p] = o.f.first[p];
         o.f.first[p + 1] = uint16_t(o.f.first[p] + count[p]);   // at most kObsMaxTerms
     }
@@ -1170,11 +1174,21 @@ struct ObsRun {
     unsigned count;
     double value() const
     {
-        double acc = 0.0;
+        // up to a thousand of them, one after the other: in extended precision, so that
+        // the number of CTAs does not show in the rounding
+        long double acc = 0.0L;
         for (unsigned b = 0; b < count; ++b) acc += partial[b];
-        return acc;
+        return double(acc);
     }
 };
+
+// States that take k_obs<0>: while its CTAs (one per 256 amplitudes) are few per SM,
+// each thread's walk over the terms is the time of <O>, and k_obs<4> shares that walk
+// among 16 amplitudes that are not there to share it.  12 qubits, 14 and 1000 terms:
+// 21 and 52 us, k_obs<4> 30 and 83; 16 qubits 21 and 76, 30 and 75; 17 qubits 23 and
+// 117, 30 and 75 (60 terms: 30 either way); 18 qubits, 200 terms 57, 37.
+constexpr uint32_t kObsNarrowQubits = 17;
+constexpr size_t kObsNarrowTerms = 64;   // at 17 qubits
 
 // Enqueues <psi|O|psi> (and lam = O psi if lam != nullptr).  The caller
 // synchronises before host_small is used again.
@@ -1184,7 +1198,8 @@ ObsRun launch_obs(qse_state* st, const qse_observable* obs, double2* lam)
     qse_ctx* ctx = st->ctx;
     if (obs->nterms > kObsMaxTerms) fail(QSE_ERR_SIZE, "observable has too many terms");
     const uint64_t size = st->size();
-    const uint64_t chunks = (size + uint64_t(kRB) * kObsR - 1) / (uint64_t(kRB) * kObsR);
+    const uint32_t bits = st->n > kObsNarrowQubits || (st->n == kObsNarrowQubits && obs->nterms > kObsNarrowTerms) ? kObsBits : 0;
+    const uint64_t chunks = (size + (uint64_t(kRB) << bits) - 1) / (uint64_t(kRB) << bits);
     const unsigned grid = unsigned(std::min<uint64_t>(chunks, uint64_t(ctx->num_sms) * 8));
     size_t obytes = align16(16 * obs->nterms);
     QSE_CUDA(cudaEventSynchronize(ctx->small_event));   // host_small may still feed an earlier copy
@@ -1192,13 +1207,14 @@ ObsRun launch_obs(qse_state* st, const qse_observable* obs, double2* lam)
     ctx->host_small.reserve(obytes + size_t(grid) * 8 + 16);
     char* d = static_cast<char*>(ctx->scratch.ptr);
     char* h = static_cast<char*>(ctx->host_small.ptr);
-    ObsDev o = upload_obs(st, obs, d, h);
+    ObsDev o = upload_obs(st, obs, bits, d, h);
     QSE_CUDA(cudaEventRecord(ctx->small_event, ctx->stream));
     double* partial = reinterpret_cast<double*>(d + obytes);
     const size_t smem = 16 * obs->nterms;
+    const auto kernel = bits ? k_obs<kObsBits> : k_obs<0>;
     if (smem > 47 * 1024)   // beyond what a launch gets unasked: 48 KiB, some of it the kernel's static arrays
-        QSE_CUDA(cudaFuncSetAttribute(k_obs, cudaFuncAttributeMaxDynamicSharedMemorySize, int(16 * kObsMaxTerms)));
-    k_obs<<<grid, kRB, smem, ctx->stream>>>(reinterpret_cast<const double2*>(st->amp), lam, size, o.z, o.w,
+        QSE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(16 * kObsMaxTerms)));
+    kernel<<<grid, kRB, smem, ctx->stream>>>(reinterpret_cast<const double2*>(st->amp), lam, size, o.z, o.w,
                                                         o.nt, o.f, o.c, partial);
     QSE_CUDA(cudaGetLastError());
     count_launch(ctx);

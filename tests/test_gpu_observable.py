@@ -86,3 +86,36 @@ def test_gradient_with_as_many_terms_as_are_accepted():
     vw, gw = O.adjoint(n, ops, params, obs)
     assert abs(v - vw) <= 1e-10
     assert np.max(np.abs(g - gw)) <= 1e-10
+
+
+# one amplitude per thread up to 17 qubits, 16 above, and at 17 qubits from 65 terms on
+@pytest.mark.parametrize("n,nterms", [(4, 100), (16, 64), (16, 65), (17, 0), (17, 64), (17, 65), (17, 300), (18, 5)])
+def test_either_side_of_the_kernels(n, nterms):
+    from quantumsimevo_b200.circuit import Circuit
+
+    rng = np.random.default_rng(100 * n + nterms)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    psi /= np.linalg.norm(psi)
+    c = Circuit(n)
+    c.state.upload(psi)
+    z = rng.integers(0, 1 << n, nterms, dtype=np.uint64)
+    w = rng.standard_normal(nterms)
+    # some hundred terms added one by one: as many roundings of 2^-53 of sum |w|, with the norm 1
+    assert abs(c.expectation(z, w, 0.25) - _plain(psi, z, w, 0.25)) <= 1e-13 * (0.25 + float(np.abs(w).sum()))
+
+
+@pytest.mark.parametrize("n", [16, 17, 18])
+def test_gradient_on_either_side(n):
+    import oracle_ffi as O
+    from quantumsimevo_b200 import _lib as L
+    from quantumsimevo_b200.autograd import ParametrizedCircuit
+
+    ops = np.zeros(2 * n, dtype=L.OP_DTYPE)
+    ops["type"], ops["target"], ops["param"], ops["coeff"] = [L.RY, L.RX] * n, np.arange(2 * n) // 2, np.arange(2 * n), 1.0
+    params = np.random.default_rng(n).uniform(-3, 3, 2 * n)
+    z, w = [(1 << q) | 1 for q in range(1, n)] + [1 << (n - 1)], list(np.linspace(-1, 1, n))
+    v, g = ParametrizedCircuit(n, ops, z, w, 0.5).value_and_grad(params)
+    obs, keep = L.observable(z, w, 0.5)
+    vw, gw = O.adjoint(n, ops, params, obs)
+    assert abs(v - vw) <= 1e-10
+    assert np.max(np.abs(g - gw)) <= 1e-10
