@@ -1219,7 +1219,9 @@ __device__ __forceinline__ uint64_t lower_bound_dev(const double* a, uint64_t n,
 // such block rebuilds its exact cumulative values in shared memory
 // (block_exact, the reference's sequential rounding) and answers its shots
 // there.  A million shots on 2^30 random amplitudes: 4.5 ms when every block
-// that holds a shot is rebuilt (98 % of them).
+// that holds a shot is rebuilt (98 % of them).  With many shots to a block all
+// of them are bucketed, without a search by a warp each: a block is rebuilt once
+// for all its shots.
 
 // The first b in [lo, lo + len) with !(cin[b + 1] < t), else lo + len.  The whole
 // warp searches, 32 probes a round.
@@ -1238,8 +1240,40 @@ __device__ __forceinline__ uint32_t warp_find_block(const double* __restrict__ c
     return lo;
 }
 
-// target = u * total (StateVector.cpp:100-107's uniform_real_distribution(0, total));
-// targets beyond the total answer size.  One warp per shot; blk[s] = nb for a
+// target = u * total (StateVector.cpp:100-107's uniform_real_distribution(0, total))
+__device__ __forceinline__ double shot_target(const double* __restrict__ u, uint64_t s, uint64_t seed, double total)
+{
+    double us;
+    if (u) us = u[s];
+    else {
+        double u2;
+        philox_uniform_pair(seed, s, kTagSample, us, u2);
+    }
+    return __dadd_rn(__dmul_rn(us, total), 0.0);
+}
+
+// Every shot to its block, the first b with cin[b + 1] >= its target; targets
+// beyond the total answer size.  One thread per shot.
+__global__ void __launch_bounds__(256) k_shot_block(const double* __restrict__ cin, uint32_t nb,
+                                                    const double* __restrict__ u, uint64_t nshots, uint64_t seed,
+                                                    uint64_t size, double* __restrict__ target, uint32_t* __restrict__ blk,
+                                                    uint32_t* __restrict__ count, uint64_t* __restrict__ out)
+{
+    const double total = cin[nb];
+    for (uint64_t s = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; s < nshots; s += uint64_t(gridDim.x) * blockDim.x) {
+        const double t = shot_target(u, s, seed, total);
+        const uint32_t b = uint32_t(lower_bound_dev(cin + 1, nb, t));
+        blk[s] = b;
+        if (b >= nb) {
+            out[s] = size;   // beyond the end: lower_bound returns size
+        } else {
+            target[s] = t;
+            atomicAdd(count + b, 1u);
+        }
+    }
+}
+
+// The same, and most shots answered at once.  One warp per shot; blk[s] = nb for a
 // shot answered here, else its block (counted for the bucketing).  Bound by the
 // L2's 32-byte sectors: a round of probes touches 32 of them, as many as half a
 // slice, so the first rounds go through a table of every nb / kTop-th block end
@@ -1260,13 +1294,7 @@ __global__ void __launch_bounds__(256) k_shot_direct(const double* __restrict__ 
     for (uint32_t i = threadIdx.x; i < ntop; i += blockDim.x) top[i] = cin[min((i + 1) * stride, nb)];
     __syncthreads();
     for (uint64_t s = blockIdx.x * uint64_t(blockDim.x >> 5) + (threadIdx.x >> 5); s < nshots; s += nwarps) {
-        double us;
-        if (u) us = u[s];
-        else {
-            double u2;
-            philox_uniform_pair(seed, s, kTagSample, us, u2);
-        }
-        const double t = __dadd_rn(__dmul_rn(us, total), 0.0);
+        const double t = shot_target(u, s, seed, total);
         uint32_t seg = 0, len = ntop;
         while (len > 0) {
             const uint32_t half = len >> 1, mid = seg + half;
@@ -1482,6 +1510,12 @@ __global__ void __launch_bounds__(kBT) k_search_each(const double* __restrict__ 
 }
 constexpr size_t kEachSmem = (size_t(kBT) * kPad + kBS) * sizeof(double);
 constexpr size_t kFewShots = 64;
+// From this many shots per block of the state on, all are bucketed: a warp per shot
+// takes 0.74 us per thousand shots, a rebuilt block about 0.02 us once it is shared.
+// On Gaussian amplitudes (buckets, else a warp each): 22 qubits, 50 000 shots 82 us
+// (105); 24 qubits, 100 000 139 (144); 25 qubits, 200 000 223 (223); 26 qubits,
+// 400 000 394 (387), a million 442 (842).
+constexpr size_t kShotsPerBlock = 24;
 
 // shared memory of k_block_search: two staging buffers + one block's cumulative values
 constexpr size_t kSearchSmem = kStage2 + size_t(kBS) * sizeof(double);
@@ -1790,9 +1824,13 @@ void sample_on(qse_state* st, const CdfView& v, const double* d_u, size_t nshots
     uint32_t* pnz = reinterpret_cast<uint32_t*>(take(size_t(nchunks) * 4));
     // count and cursor are adjacent: one clear
     QSE_CUDA(cudaMemsetAsync(count, 0, reinterpret_cast<char*>(offset) - reinterpret_cast<char*>(count), ctx->stream));
-    const unsigned wgrid = unsigned(std::min<uint64_t>((nshots + 7) / 8, uint64_t(ctx->num_sms) * 8));
-    k_shot_direct<<<wgrid, 256, 0, ctx->stream>>>(v.cin, nb, v.cdf, v.slices(), v.slice_e(), d_u, nshots, seed,
-                                                  st->size(), target, blk, count, d_out);
+    if (nshots / kShotsPerBlock >= nb) {
+        k_shot_block<<<grid, 256, 0, ctx->stream>>>(v.cin, nb, d_u, nshots, seed, st->size(), target, blk, count, d_out);
+    } else {
+        const unsigned wgrid = unsigned(std::min<uint64_t>((nshots + 7) / 8, uint64_t(ctx->num_sms) * 8));
+        k_shot_direct<<<wgrid, 256, 0, ctx->stream>>>(v.cin, nb, v.cdf, v.slices(), v.slice_e(), d_u, nshots, seed,
+                                                      st->size(), target, blk, count, d_out);
+    }
     k_scan_part<<<nchunks, kOT, 0, ctx->stream>>>(count, nb, psum, pnz);
     k_scan_top<<<1, kOT, 0, ctx->stream>>>(psum, pnz, nchunks, offset + nb, nne);
     k_scan_final<<<nchunks, kOT, 0, ctx->stream>>>(count, nb, psum, pnz, offset, nonempty);

@@ -57,3 +57,30 @@ def test_sample_bit_exact_across_binades(n, kind, few):
     u = np.ascontiguousarray(u)
     L.check(L.lib.qse_sample(st.handle, u.ctypes.data_as(L._pd), len(u), 0, out.ctypes.data_as(L._pu64)))
     assert np.array_equal(out, O.sample(amp, n, u))
+
+
+# 24 shots per 4096-amplitude block and more are bucketed by block, fewer answered a warp each
+@pytest.mark.parametrize("kind", ["zero prefix", "growing", "ties", "ties then jump", "subnormal", "uniform", "random"])
+@pytest.mark.parametrize("n", [14, 15, 17])
+def test_few_and_many_shots_per_block(n, kind):
+    size = 1 << n
+    rng = np.random.default_rng(11 * n + len(kind))
+    amp = _amplitudes(kind, size, rng)
+    cum = np.asarray(O.cdf(amp, n))
+    limit = 24 * (size // 4096)
+    at = rng.integers(0, size, limit)
+    u = cum[at] / cum[-1]
+    u[::3] = np.nextafter(u[::3], 0.0)
+    u[1::3] = rng.random(len(u[1::3]))
+    u = np.clip(u, 0.0, np.nextafter(1.0, 0.0))
+    st = StateVector(n)
+    st.upload(amp)
+    want = O.sample(amp, n, u)
+    for shots in (limit - 1, limit):
+        out = np.empty(shots, dtype=np.uint64)
+        L.check(L.lib.qse_sample(st.handle, u.ctypes.data_as(L._pd), shots, 0, out.ctypes.data_as(L._pu64)))
+        assert np.array_equal(out, want[:shots])
+    drawn = np.empty((2, limit), dtype=np.uint64)   # the device's own draws: the same on either route
+    L.check(L.lib.qse_sample(st.handle, None, limit - 1, 5, drawn[0].ctypes.data_as(L._pu64)))
+    L.check(L.lib.qse_sample(st.handle, None, limit, 5, drawn[1].ctypes.data_as(L._pu64)))
+    assert np.array_equal(drawn[0, : limit - 1], drawn[1, : limit - 1])
