@@ -826,6 +826,14 @@ constexpr uint32_t kLowLanesQubits = 23;
 // gain below.
 constexpr uint32_t kLaneSwapQubits = 20;
 
+// Reverse passes of states of at least this many qubits hold 16 amplitudes of each
+// state per thread, below it 8, whose code is half as long to compile and to fetch.
+// Gradients, 8 and 16 per thread: HEA of 10 layers, 11 qubits 231 and 278 us (first
+// run 10.2 and 14.9 s), 18 qubits 475 and 521 us, 21 qubits 1.61 and 1.63 ms, 22
+// qubits 3.40 and 3.33, 24 qubits 12.8 and 12.3; QAOA of 3 layers, 21 qubits 465 and
+// 507 us, 22 qubits 976 and 1020, 24 qubits 3.19 and 3.09 ms.
+constexpr uint32_t kAdjoint16Qubits = 22;
+
 uint32_t tile_size(int tile_qubits, uint32_t n, uint32_t rb, uint32_t kmax)
 {
     return std::min(std::min<uint32_t>(std::max(tile_qubits, int(rb) + 1), kmax), n);
@@ -862,11 +870,11 @@ Options adjoint_options(const Settings& s, uint32_t n)
 {
     Options opt;
     opt.k = tile_size(s.tile_qubits, n, 3, 11);
-    // specialised kernels hold 16 amplitudes of both states per thread: the
-    // register shape of the forward passes (128 threads, three CTAs per SM), half
-    // the barriers of 8 per thread, and a layout exchange per four register
-    // qubits instead of three (passes of a 24-qubit QAOA: 452 -> 373 us)
-    opt.rb = s.jit && opt.k == 11 ? 4 : 3;
+    // on large states specialised kernels hold 16 amplitudes of both states per
+    // thread: the register shape of the forward passes (128 threads, three CTAs per
+    // SM), half the barriers of 8 per thread, and a layout exchange per four
+    // register qubits instead of three (passes of a 24-qubit QAOA: 452 -> 373 us)
+    opt.rb = s.jit && opt.k == 11 && n >= kAdjoint16Qubits ? 4 : 3;
     opt.grads = true;
     opt.max_terms = 512;
     opt.max_gates = kJitMaxGates;

@@ -48,7 +48,7 @@ def test_first_pass_from_a_compact_state(tmp_path, monkeypatch):
     assert {amplitudes(t) for f, t in k.items() if not f.startswith("qse_pass_compact_in")} == {16}
 
 
-@pytest.mark.parametrize("n,amps,swaps", [(10, 8, False), (11, 16, False), (19, 16, False), (20, 16, True), (24, 16, True)])
+@pytest.mark.parametrize("n,amps,swaps", [(10, 8, False), (11, 8, False), (19, 8, False), (20, 8, True), (22, 16, True), (24, 16, True)])
 def test_reverse_passes(tmp_path, monkeypatch, n, amps, swaps):
     ops, params, _, _ = W.qaoa_maxcut(n if n % 2 == 0 else n + 1, 1, seed=3)
     ops = ops[(ops["target"] < n) & (ops["control"] < n)]
