@@ -61,7 +61,7 @@ def test_sample_bit_exact_across_binades(n, kind, few):
 
 # 24 shots per 4096-amplitude block and more are bucketed by block, fewer answered a warp each
 @pytest.mark.parametrize("kind", ["zero prefix", "growing", "ties", "ties then jump", "subnormal", "uniform", "random"])
-@pytest.mark.parametrize("n", [14, 15, 17])
+@pytest.mark.parametrize("n", [14, 15, 17, 21])   # 21: more blocks than thread blocks rebuild at a time
 def test_few_and_many_shots_per_block(n, kind):
     size = 1 << n
     rng = np.random.default_rng(11 * n + len(kind))
