@@ -71,7 +71,7 @@ def expect(where, threads, states, got):
 
 
 @pytest.mark.parametrize("where", ["load", "store", "both", "neither"])
-@pytest.mark.parametrize("n,k", [(20, 8), (20, 9), (20, 10), (20, 12), (21, 11), (22, 12)])
+@pytest.mark.parametrize("n,k", [(20, 8), (20, 9), (20, 10), (20, 12), (21, 11), (22, 12), (23, 12)])
 def test_one_state(n, k, where, tmp_path, monkeypatch):
     monkeypatch.setenv("QSE_JIT_DUMP", str(tmp_path))
     dev = Device(0)
